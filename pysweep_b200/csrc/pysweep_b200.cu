@@ -16,6 +16,7 @@
 #include "swept.cuh"
 #include "heat_fast.cuh"
 #include "seam_fast.cuh"
+#include "heat_block.cuh"
 #include "standard_fast.cuh"
 #include "euler_faces.cuh"
 #include "batch.cuh"
@@ -74,6 +75,7 @@ struct ps_solver {
     // Laplacians (ps_set_field; device memory the caller owns)
     double* field[3] = {nullptr, nullptr, nullptr};
     bool nseg_auto = true;  // choose the segment count per run until configured
+    bool h_set = false;     // levels per half-cycle configured
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     // the gap stream runs beside the y-bridge seam on a high-priority side
@@ -384,7 +386,7 @@ cudaEvent_t take_event(ps_solver* s)
 }
 
 // Kernel kinds for ps_profile_read: 0 prism stream, 1 Y-bridge seam, 2 gap
-// stream, 3 octahedron seam, 4 standard step.
+// stream, 3 octahedron seam, 4 standard step, 5 overlapped block.
 template <class F>
 int timed_launch(ps_solver* s, int kind, double cells, F&& launch, cudaStream_t st = nullptr)
 {
@@ -543,6 +545,169 @@ int hook_frame(ps_solver* s, int ns, int rows, int cols, int times)
     return PS_OK;
 }
 
+// ------------------------------------------------- overlapped heat blocks ----
+// A kernel that may begin while the one before it in the stream ends (it waits
+// for it itself: grid_wait).
+template <class... A>
+void launch_after(void (*k)(A...), int grid, int nt, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(nt);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, args...);
+}
+
+template <class S, bool RK2, int C, int R, int MAXW>
+void launch_tile(const BlockArgs& a, int nw, cudaStream_t st)
+{
+    auto k = heat_block_tile<S, RK2, C, R, MAXW>;
+    const size_t smem = tile_smem<C>(nw);
+    if (smem > 48 * 1024) allow_big_smem(k);
+    launch_after(k, a.units, 32 * nw, smem, st, a);
+}
+
+template <class S, bool RK2>
+void launch_block_tile(const TileShape& t, BlockArgs a, int T, cudaStream_t st)
+{
+    a.T = T;
+    a.vw = tile_vw(t, T);
+    a.vh = tile_vh(t, T);
+    a.ncs = (a.ny + a.vw - 1) / a.vw;
+    a.units = a.ncs * ((a.nx + a.vh - 1) / a.vh);
+    if constexpr (RK2) {
+        if (t.C == 4) launch_tile<S, RK2, 4, 4, 16>(a, t.nw, st);
+        else launch_tile<S, RK2, 2, 4, 24>(a, t.nw, st);
+    } else {
+        if (t.C == 4) launch_tile<S, RK2, 4, 6, 16>(a, t.nw, st);
+        else if (t.R == 8) launch_tile<S, RK2, 2, 8, 20>(a, t.nw, st);
+        else launch_tile<S, RK2, 2, 4, 24>(a, t.nw, st);
+    }
+}
+
+template <class S, bool RK2>
+void launch_block_stream(BlockArgs a, int sms, cudaStream_t st)
+{
+    a.T = kStreamT;
+    a.vw = kStreamW;
+    a.ncs = (a.ny + a.vw - 1) / a.vw;
+    a.vh = stream_rows(a.nx, a.ny, sms);
+    a.units = a.ncs * ((a.nx + a.vh - 1) / a.vh);
+    launch_after(heat_block_stream<S, RK2>, a.units, 32, 0, st, a);
+}
+
+bool aligned32(const void* p) { return reinterpret_cast<uintptr_t>(p) % 32 == 0; }
+
+// Heat through overlapped space-time blocks (heat_block.cuh): forward Euler
+// with its 1, or the two-stage scheme with its 2.  maxT: levels per launch at
+// most.  Two-stage levels run in pairs from a half stage on; a level left over
+// on either side (a run that begins with a full stage, an odd count) is one
+// standard step.
+template <class S, bool RK2>
+int run_block(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t frame_cap,
+              int frame_every, int maxT)
+{
+    constexpr int step = RK2 ? 2 : 1;
+    const size_t fe = field_elems(s);
+    const int its = s->its;
+    const int every = frame_every > 0 ? frame_every : 1;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
+    const EqParams prm = make_params(s);
+    auto frame_of = [&](int64_t L) -> double* {
+        if (!frames || L % its || (L / its) % every) return nullptr;
+        const int64_t slot = (L / its) / every - 1;
+        return slot < frame_cap ? at(s, frames, (size_t)slot * fe) : nullptr;
+    };
+    auto newest = [&](int b) { return at(s, s->base[b], (size_t)(its - 1) * fe); };
+    int rc;
+    int64_t done = 0;
+    auto single = [&]() -> int {  // one level of the two-stage scheme
+        const int b = s->cur;
+        double* fr = frame_of(done + 1);
+        const int gts = gts0 + (int)done;
+        if (int e = timed_launch(s, 4, (double)s->nx * s->ny, [&] {
+                launch_standard<Heat>(newest(b), s->base[b], newest(1 - b), fr, s->nx, s->ny, 1,
+                                      gts, prm, s->stream);
+            }))
+            return e;
+        PS_CUDA(s, cudaMemcpyAsync(s->base[1 - b], newest(b), nbytes(s, fe),
+                                   cudaMemcpyDeviceToDevice, s->stream));
+        s->cur = 1 - b;
+        ++done;
+        return PS_OK;
+    };
+    if (RK2 && nlevels > 0 && gts0 % 2 == 0 && (rc = single())) return rc;
+    const int64_t last = RK2 ? nlevels - (nlevels - done) % 2 : nlevels;
+    auto plan_for = [&](int64_t n) {
+        const int m = (int)std::min<int64_t>(n, 1 << 20);
+        if constexpr (RK2) return plan_block(kTilesRK2, s->nx, s->ny, m, step, maxT, sms);
+        else return plan_block(kTilesFE, s->nx, s->ny, m, step, maxT, sms);
+    };
+    BlockPlan plan{};
+    BlockArgs a;
+    memset(&a, 0, sizeof a);
+    a.nx = s->nx;
+    a.ny = s->ny;
+    a.v4 = s->ny % 4 == 0;
+    a.cr = prm.d[0];
+    if (done < last) plan = plan_for(last - done);
+    // frames are stored by the block that computes their level where 4-wide
+    // stores may reach them; else the block ends at the level and it is copied
+    const bool direct = aligned32(frames);
+    while (done < last) {
+        const int64_t left = last - done;
+        const bool stream = plan.stream && left >= kStreamT;
+        int T = stream ? kStreamT : (int)std::min<int64_t>(plan.T, left);
+        if (!plan.stream) {  // even shares over the launches left
+            const int64_t k = (left + plan.T - 1) / plan.T;
+            T = (int)(((left + k - 1) / k + step - 1) / step * step);
+        }
+        a.nframe = 0;
+        double* copy_to = nullptr;
+        for (int m = 1; m <= T; ++m) {
+            double* f = frame_of(done + m);
+            a.frame[m - 1] = direct ? f : nullptr;
+            if (f && direct) ++a.nframe;
+            if (f && !direct) {
+                copy_to = f;
+                T = m;
+            }
+        }
+        a.in = newest(s->cur);
+        a.out = newest(1 - s->cur);
+        // the level before the newest is part of the state after the run
+        a.out1 = RK2 && done + T == nlevels ? s->base[1 - s->cur] : nullptr;
+        // frames and the kept level are stored by the tiles only
+        const bool tile = !stream || T < kStreamT || a.nframe || a.out1;
+        if ((rc = timed_launch(s, 5, (double)s->nx * s->ny * T, [&] {
+                 if (tile) {
+                     double us;
+                     if constexpr (RK2)
+                         launch_block_tile<S, RK2>(best_tile(kTilesRK2, T, s->nx, s->ny, sms, &us), a, T, s->stream);
+                     else
+                         launch_block_tile<S, RK2>(best_tile(kTilesFE, T, s->nx, s->ny, sms, &us), a, T, s->stream);
+                 } else {
+                     launch_block_stream<S, RK2>(a, sms, s->stream);
+                 }
+             })))
+            return rc;
+        s->cur = 1 - s->cur;
+        done += T;
+        if (copy_to)
+            PS_CUDA(s, cudaMemcpyAsync(copy_to, newest(s->cur), nbytes(s, fe),
+                                       cudaMemcpyDeviceToDevice, s->stream));
+    }
+    if (done < nlevels && (rc = single())) return rc;
+    return PS_OK;
+}
+
 int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t frame_cap,
               int frame_every)
 {
@@ -647,6 +812,18 @@ int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
     const size_t smem = std::max(stream_smem(s), seam_smem(s));
     if (smem > 227 * 1024)
         return fail(s, PS_ERR_UNSUPPORTED, "tile needs %zu bytes of shared memory", smem);
+    // heat in overlapped blocks; threads 256 keeps the shared-memory prisms,
+    // and a configured h bounds the levels of a launch
+    if (!s->hook && s->eq == PS_EQ_HEAT && s->threads != 256 && (s->its == 1) == fwd_euler) {
+        const int maxT = s->h_set ? s->H : kTileMaxT;
+        if (s->dtype == PS_DTYPE_F32)
+            return run_block<float, false>(s, nlevels, gts0, frames, frame_cap, frame_every, maxT);
+        if (fwd_euler)
+            return run_block<double, false>(s, nlevels, gts0, frames, frame_cap, frame_every, maxT);
+        // (frames that 4-wide stores cannot reach may fall on half stages)
+        if (maxT >= 2 && aligned32(frames))
+            return run_block<double, true>(s, nlevels, gts0, frames, frame_cap, frame_every, maxT);
+    }
     int rc = ensure_swept_buffers(s);
     if (rc) return rc;
     if (!s->side) {
@@ -1253,6 +1430,7 @@ int ps_configure(ps_solver* s, int h, int nseg, int chunk, int threads)
     if (h) {
         if (h > s->mpss) return fail(s, PS_ERR_INVALID, "h %d > MPSS %d", h, s->mpss);
         s->H = h;
+        s->h_set = true;
     }
     if (nseg) {
         s->nseg = nseg;

@@ -219,7 +219,7 @@ class Engine:
     def synchronize(self):
         check(_lib.lib().ps_synchronize(self._h), self._h)
 
-    KINDS = ("prism", "ybridge", "gap", "octahedron", "standard")
+    KINDS = ("prism", "ybridge", "gap", "octahedron", "standard", "block")
 
     def profile(self, enable=True):
         """Bracket every following launch with CUDA events (resets the counters)."""
