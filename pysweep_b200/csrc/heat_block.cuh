@@ -449,18 +449,39 @@ struct BlockPlan {
 inline int tile_vw(const TileShape& t, int T) { return 32 * t.C - 2 * ((T + t.C - 1) / t.C * t.C); }
 inline int tile_vh(const TileShape& t, int T) { return t.nw * t.R - 2 * T; }
 
+// The grids of one launch: a solver's one, a batch's many.
+struct BlockGrid {
+    int nx, ny;
+};
+struct BlockGrids {
+    const BlockGrid* g;
+    int n;
+    long long blocks(int vw, int vh) const
+    {
+        long long k = 0;
+        for (int i = 0; i < n; ++i)
+            k += (long long)((g[i].ny + vw - 1) / vw) * ((g[i].nx + vh - 1) / vh);
+        return k;
+    }
+    int rows() const
+    {
+        int m = 1;
+        for (int i = 0; i < n; ++i) m = std::max(m, g[i].nx);
+        return m;
+    }
+};
+
 // Estimated microseconds of one launch of T levels in tiles of shape t, or 0
 // where no cell of the tile stays exact.  Fitted to launches of 160² to 8192²
 // (within 15%): a level of one tile takes its FP64 operations at the pipe's
 // rate (16 cycles per warp and cell) and, with few warps on the SM, the latency
 // of the exchange; loading and storing cost 0.03 us per KB of the tiles on an
 // SM, hidden behind other tiles where the SM holds more than one.
-inline double tile_us(const TileShape& t, int T, int nx, int ny, int sms)
+inline double tile_us(const TileShape& t, int T, const BlockGrids& g, int sms)
 {
     const int vw = tile_vw(t, T), vh = tile_vh(t, T);
     if (vw < 8 || vh < 2) return 0.0;
-    const long long tiles = (long long)((ny + vw - 1) / vw) * ((nx + vh - 1) / vh);
-    const double n = (double)((tiles + sms - 1) / sms);  // tiles of the busiest SM
+    const double n = (double)((g.blocks(vw, vh) + sms - 1) / sms);  // tiles of the busiest SM
     const int occ = t.maxw / t.nw;
     const double k = std::min(n, (double)occ), rounds = std::max(1.0, n / occ);
     const double level = 4.0 * t.nw * t.R * t.C / 1965.0 * 1.04;
@@ -469,23 +490,28 @@ inline double tile_us(const TileShape& t, int T, int nx, int ny, int sms)
     return 1.0 + n * T * level + (occ == 1 ? rounds : 1.0) * kb + (n - k) * 0.4 + lat * T * rounds;
 }
 
-// Rows of a stream's strip: one wave of eight warps per SM.
-inline int stream_rows(int nx, int ny, int sms)
+// Rows of a stream's strip: the fewest that fill no more than one wave of
+// eight warps per SM (the whole grid's where even those make more strips).
+inline int stream_rows(const BlockGrids& g, int sms)
 {
-    const int ncs = (ny + kStreamW - 1) / kStreamW;
-    const int rs = std::max(1, std::min(nx, 8 * sms / ncs));
-    return (nx + rs - 1) / rs;
+    int lo = 1, hi = g.rows();
+    while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (g.blocks(kStreamW, mid) <= 8LL * sms) hi = mid;
+        else lo = mid + 1;
+    }
+    return lo;
 }
 
 // The cheapest tile for one launch of T levels.
 template <int NSHAPE>
-inline TileShape best_tile(const TileShape (&shapes)[NSHAPE], int T, int nx, int ny, int sms,
+inline TileShape best_tile(const TileShape (&shapes)[NSHAPE], int T, const BlockGrids& g, int sms,
                            double* us)
 {
     TileShape best = shapes[0];
     *us = 1e300;
     for (const TileShape& t : shapes) {
-        const double one = tile_us(t, T, nx, ny, sms);
+        const double one = tile_us(t, T, g, sms);
         if (one > 0 && one < *us) {
             *us = one;
             best = t;
@@ -499,27 +525,89 @@ inline TileShape best_tile(const TileShape (&shapes)[NSHAPE], int T, int nx, int
 // 4096² 11.6 / 15.7, 8192² 42.4 / 60.0); below, the tile whose count fits the
 // SMs best.
 template <int NSHAPE>
-inline BlockPlan plan_block(const TileShape (&shapes)[NSHAPE], int nx, int ny, int nlevels, int step,
-                            int maxT, int sms)
+inline BlockPlan plan_block(const TileShape (&shapes)[NSHAPE], const BlockGrids& g, int nlevels,
+                            int step, int maxT, int sms)
 {
     BlockPlan best{false, step, 1e300};
     for (int T = step; T <= std::min(maxT, kTileMaxT); T += step) {
         const int k = (nlevels + T - 1) / T;
         const int Tk = ((nlevels + k - 1) / k + step - 1) / step * step;  // even shares
         double one;
-        best_tile(shapes, Tk, nx, ny, sms, &one);
+        best_tile(shapes, Tk, g, sms, &one);
         if (k * one < best.us) best = BlockPlan{false, Tk, k * one};
     }
     if (nlevels >= kStreamT && maxT >= kStreamT) {
-        const int ncs = (ny + kStreamW - 1) / kStreamW, rows = stream_rows(nx, ny, sms);
-        // (strips of very wide grids may fill more than one wave)
-        const double waves = std::max(1.0, (double)ncs * ((nx + rows - 1) / rows) / (8.0 * sms));
+        const int rows = stream_rows(g, sms);
+        // (strips of very wide grids, or of many, may fill more than one wave)
+        const double waves = std::max(1.0, (double)g.blocks(kStreamW, rows) / (8.0 * sms));
         double us = nlevels / kStreamT * (10.2 + 0.645 * rows) * waves, tail = 0.0;
         const int rest = (nlevels % kStreamT + step - 1) / step * step;
-        if (rest) best_tile(shapes, rest, nx, ny, sms, &tail);
+        if (rest) best_tile(shapes, rest, g, sms, &tail);
         if (us + tail < best.us) best = BlockPlan{true, kStreamT, us + tail};
     }
     return best;
+}
+
+// Levels of the next launch with `left` levels to go: streams while there are
+// enough, tiles in even shares.
+inline int plan_next(const BlockPlan& p, long long left, int step)
+{
+    if (p.stream) return left >= kStreamT ? kStreamT : (int)((left + step - 1) / step * step);
+    const long long k = (left + p.T - 1) / p.T;
+    return (int)(((left + k - 1) / k + step - 1) / step * step);
+}
+
+// ------------------------------------------------------------------ batch --
+// Many grids in one launch: block g is unit units[g].y of grid units[g].x.
+struct BlockInst {
+    double* base[2];
+    double cr;
+    int nx, ny;
+};
+
+__device__ __forceinline__ void batch_block_args(const BlockInst* inst, int i, int par, int T,
+                                                 int vw, int vh, BlockArgs& a)
+{
+    const BlockInst b = inst[i];
+    a.in = b.base[par];
+    a.out = b.base[1 - par];
+    a.out1 = nullptr;
+    a.nx = b.nx;
+    a.ny = b.ny;
+    a.T = T;
+    a.vw = vw;
+    a.vh = vh;
+    a.ncs = (b.ny + vw - 1) / vw;
+    a.units = 0;
+    a.v4 = b.ny % 4 == 0;
+    a.nframe = 0;
+    a.cr = b.cr;
+}
+
+__global__ void __launch_bounds__(32, 8)
+    heat_block_stream_batch(const BlockInst* __restrict__ inst, const int2* __restrict__ units,
+                            int par, int vh)
+{
+    __shared__ __align__(16) double ring[kBlockRing * 32 * kStreamC];
+    const int2 u = units[blockIdx.x];
+    BlockArgs a;
+    batch_block_args(inst, u.x, par, kStreamT, kStreamW, vh, a);
+    grid_wait();
+    grid_release();
+    block_stream_body<double, false>(a, u.y, ring);
+}
+
+template <int C, int R, int MAXW>
+__global__ void __launch_bounds__(32 * MAXW, 1)
+    heat_block_tile_batch(const BlockInst* __restrict__ inst, const int2* __restrict__ units,
+                          int par, int T, int vw, int vh)
+{
+    extern __shared__ __align__(16) double tile_sm[];
+    const int2 u = units[blockIdx.x];
+    BlockArgs a;
+    batch_block_args(inst, u.x, par, T, vw, vh, a);
+    grid_wait();
+    block_tile_body<double, false, C, R>(a, u.y, blockDim.x >> 5, tile_sm);
 }
 
 }  // namespace psb

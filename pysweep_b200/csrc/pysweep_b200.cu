@@ -597,7 +597,8 @@ void launch_block_stream(BlockArgs a, int sms, cudaStream_t st)
     a.T = kStreamT;
     a.vw = kStreamW;
     a.ncs = (a.ny + a.vw - 1) / a.vw;
-    a.vh = stream_rows(a.nx, a.ny, sms);
+    const BlockGrid g{a.nx, a.ny};
+    a.vh = stream_rows(BlockGrids{&g, 1}, sms);
     a.units = a.ncs * ((a.nx + a.vh - 1) / a.vh);
     launch_after(heat_block_stream<S, RK2>, a.units, 32, 0, st, a);
 }
@@ -645,11 +646,8 @@ int run_block(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
     };
     if (RK2 && nlevels > 0 && gts0 % 2 == 0 && (rc = single())) return rc;
     const int64_t last = RK2 ? nlevels - (nlevels - done) % 2 : nlevels;
-    auto plan_for = [&](int64_t n) {
-        const int m = (int)std::min<int64_t>(n, 1 << 20);
-        if constexpr (RK2) return plan_block(kTilesRK2, s->nx, s->ny, m, step, maxT, sms);
-        else return plan_block(kTilesFE, s->nx, s->ny, m, step, maxT, sms);
-    };
+    const BlockGrid grid{s->nx, s->ny};
+    const BlockGrids grids{&grid, 1};
     BlockPlan plan{};
     BlockArgs a;
     memset(&a, 0, sizeof a);
@@ -657,18 +655,16 @@ int run_block(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
     a.ny = s->ny;
     a.v4 = s->ny % 4 == 0;
     a.cr = prm.d[0];
-    if (done < last) plan = plan_for(last - done);
+    if (done < last) {
+        const int n = (int)std::min<int64_t>(last - done, 1 << 20);
+        if constexpr (RK2) plan = plan_block(kTilesRK2, grids, n, step, maxT, sms);
+        else plan = plan_block(kTilesFE, grids, n, step, maxT, sms);
+    }
     // frames are stored by the block that computes their level where 4-wide
     // stores may reach them; else the block ends at the level and it is copied
     const bool direct = aligned32(frames);
     while (done < last) {
-        const int64_t left = last - done;
-        const bool stream = plan.stream && left >= kStreamT;
-        int T = stream ? kStreamT : (int)std::min<int64_t>(plan.T, left);
-        if (!plan.stream) {  // even shares over the launches left
-            const int64_t k = (left + plan.T - 1) / plan.T;
-            T = (int)(((left + k - 1) / k + step - 1) / step * step);
-        }
+        int T = plan_next(plan, last - done, step);
         a.nframe = 0;
         double* copy_to = nullptr;
         for (int m = 1; m <= T; ++m) {
@@ -685,14 +681,14 @@ int run_block(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
         // the level before the newest is part of the state after the run
         a.out1 = RK2 && done + T == nlevels ? s->base[1 - s->cur] : nullptr;
         // frames and the kept level are stored by the tiles only
-        const bool tile = !stream || T < kStreamT || a.nframe || a.out1;
+        const bool tile = !plan.stream || T < kStreamT || a.nframe || a.out1;
         if ((rc = timed_launch(s, 5, (double)s->nx * s->ny * T, [&] {
                  if (tile) {
                      double us;
                      if constexpr (RK2)
-                         launch_block_tile<S, RK2>(best_tile(kTilesRK2, T, s->nx, s->ny, sms, &us), a, T, s->stream);
+                         launch_block_tile<S, RK2>(best_tile(kTilesRK2, T, grids, sms, &us), a, T, s->stream);
                      else
-                         launch_block_tile<S, RK2>(best_tile(kTilesFE, T, s->nx, s->ny, sms, &us), a, T, s->stream);
+                         launch_block_tile<S, RK2>(best_tile(kTilesFE, T, grids, sms, &us), a, T, s->stream);
                  } else {
                      launch_block_stream<S, RK2>(a, sms, s->stream);
                  }
@@ -1674,6 +1670,15 @@ struct ps_batch {
     int64_t launches = 0;
     // the instances' level counters the device descriptors were uploaded with
     std::vector<int64_t> desc_level;
+    // heat in overlapped blocks: the instances, and one table of (instance,
+    // unit) pairs per block size in use
+    BlockInst* d_binst = nullptr;
+    bool binst_current = false;
+    struct Table {
+        int vw, vh, n;
+        int2* d;
+    };
+    std::vector<Table> tables;
     std::string err;
 };
 
@@ -1779,7 +1784,6 @@ size_t batch_tile_smem(const ps_batch* b)
 
 size_t batch_stream_smem(const ps_batch* b)
 {
-    if (b->fast) return b->bs == 16 ? heat_fast_smem<16>(b->H) : heat_fast_smem<32>(b->H);
     return batch_tile_smem(b) +
            (b->faces ? sizeof(double) * euler_level_scratch(b->bs, b->chunk) : 0);
 }
@@ -1792,7 +1796,6 @@ size_t batch_seam_smem(const ps_batch* b)
                                      seam_smem_elems(true, b->bs, b->ops, b->nv, b->its, b->H));
 }
 
-using BatchFast = void (*)(const SweptArgs*, const int2*, int, int, int, long long);
 using BatchGen = void (*)(const SweptArgs*, const int2*, int, int, long long);
 
 struct BatchKernels {
@@ -1806,7 +1809,7 @@ struct BatchKernels {
 // beside G on the side stream (G reads nothing Y writes; see run_swept), then
 // O after both.
 template <class Eq, int ITS, int W>
-void batch_half(ps_batch* b, int par, int H, long long L0, size_t ssm, size_t gsm, dim3 fgrid)
+void batch_half(ps_batch* b, int par, int H, long long L0, size_t ssm, size_t gsm)
 {
     const int nu = b->nunits;
     cudaStream_t st = b->stream, sd = b->side;
@@ -1818,37 +1821,9 @@ void batch_half(ps_batch* b, int par, int H, long long L0, size_t ssm, size_t gs
         cudaEventRecord(b->ev_join, sd);
         cudaStreamWaitEvent(st, b->ev_join, 0);
     };
-    if (b->fast) {
-        if (b->bs == 16) {
-            heat_stream_fast_batch<16, false><<<fgrid, 32 * kFastWarps, gsm, st>>>(b->d_desc, b->d_units, nu, par, H, L0);
-            fork();
-            heat_stream_fast_batch<16, true><<<fgrid, 32 * kFastWarps, gsm, sd>>>(b->d_desc, b->d_units, nu, par, H, L0);
-        } else {
-            heat_stream_fast_batch<32, false><<<fgrid, 32 * kFastWarps, gsm, st>>>(b->d_desc, b->d_units, nu, par, H, L0);
-            fork();
-            heat_stream_fast_batch<32, true><<<fgrid, 32 * kFastWarps, gsm, sd>>>(b->d_desc, b->d_units, nu, par, H, L0);
-        }
-    } else {
-        stream_batch<Eq, ITS, W, false, 256><<<nu, 256, gsm, st>>>(b->d_desc, b->d_units, par, H, L0);
-        fork();
-        stream_batch<Eq, ITS, W, true, 256><<<nu, 256, gsm, sd>>>(b->d_desc, b->d_units, par, H, L0);
-    }
-    if (b->fast) {
-        // the register-resident seams, one warp per unit
-        const dim3 sgrid((nu + kSeamWarps - 1) / kSeamWarps);
-        const size_t ysm =
-            (b->bs == 16 ? yseam_smem<16>(b->H) : yseam_smem<32>(b->H)) + kSeamWarps * kDescBytes;
-        if (b->bs == 16) {
-            heat_seam_fast_batch<16, false><<<sgrid, 32 * kSeamWarps, ysm, st>>>(b->d_desc, b->d_units, nu, par, H, L0);
-            join();
-            heat_seam_fast_batch<16, true><<<sgrid, 32 * kSeamWarps, ysm, st>>>(b->d_desc, b->d_units, nu, par, H, L0);
-        } else {
-            heat_seam_fast_batch<32, false><<<sgrid, 32 * kSeamWarps, ysm, st>>>(b->d_desc, b->d_units, nu, par, H, L0);
-            join();
-            heat_seam_fast_batch<32, true><<<sgrid, 32 * kSeamWarps, ysm, st>>>(b->d_desc, b->d_units, nu, par, H, L0);
-        }
-        return;
-    }
+    stream_batch<Eq, ITS, W, false, 256><<<nu, 256, gsm, st>>>(b->d_desc, b->d_units, par, H, L0);
+    fork();
+    stream_batch<Eq, ITS, W, true, 256><<<nu, 256, gsm, sd>>>(b->d_desc, b->d_units, par, H, L0);
     seam_batch<Eq, ITS, false, 128><<<nu, 128, ssm, st>>>(b->d_desc, b->d_units, par, H, L0);
     join();
     seam_batch<Eq, ITS, true, 128><<<nu, 128, ssm, st>>>(b->d_desc, b->d_units, par, H, L0);
@@ -1857,21 +1832,13 @@ void batch_half(ps_batch* b, int par, int H, long long L0, size_t ssm, size_t gs
 template <class Eq, int ITS, int W>
 void batch_prepare()
 {
-    allow_big_smem(heat_stream_fast_batch<16, false>);
-    allow_big_smem(heat_stream_fast_batch<16, true>);
-    allow_big_smem(heat_stream_fast_batch<32, false>);
-    allow_big_smem(heat_stream_fast_batch<32, true>);
-    allow_big_smem(heat_seam_fast_batch<16, false>);
-    allow_big_smem(heat_seam_fast_batch<16, true>);
-    allow_big_smem(heat_seam_fast_batch<32, false>);
-    allow_big_smem(heat_seam_fast_batch<32, true>);
     allow_big_smem(stream_batch<Eq, ITS, W, false, 256>);
     allow_big_smem(stream_batch<Eq, ITS, W, true, 256>);
     allow_big_smem(seam_batch<Eq, ITS, false, 128>);
     allow_big_smem(seam_batch<Eq, ITS, true, 128>);
 }
 
-using HalfFn = void (*)(ps_batch*, int, int, long long, size_t, size_t, dim3);
+using HalfFn = void (*)(ps_batch*, int, int, long long, size_t, size_t);
 using PrepFn = void (*)();
 
 bool batch_pick(int eq, int ops, int its, int chunk, HalfFn* half, PrepFn* prep)
@@ -1892,14 +1859,116 @@ bool batch_pick(int eq, int ops, int its, int chunk, HalfFn* half, PrepFn* prep)
     return false;
 }
 
+// ---- heat in overlapped blocks (b->fast) ----
+struct BlockStep {
+    bool stream;
+    TileShape tile;
+    int T, table;
+};
+
+// The table of a block size, built on first use.  (Block sizes come from the
+// tile shapes and level counts, so a batch has a few hundred at most.)
+int batch_table(ps_batch* b, int vw, int vh, int* index)
+{
+    for (size_t i = 0; i < b->tables.size(); ++i)
+        if (b->tables[i].vw == vw && b->tables[i].vh == vh) {
+            *index = (int)i;
+            return PS_OK;
+        }
+    std::vector<int2> u;
+    for (int i = 0; i < (int)b->inst.size(); ++i) {
+        const BatchInst& I = b->inst[i];
+        const int n = ((I.ny + vw - 1) / vw) * ((I.nx + vh - 1) / vh);
+        for (int k = 0; k < n; ++k) u.push_back(make_int2(i, k));
+    }
+    int2* d = nullptr;
+    PSB_CUDA(b, cudaMalloc(&d, u.size() * sizeof(int2)));
+    cudaError_t e = cudaMemcpy(d, u.data(), u.size() * sizeof(int2), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+        cudaFree(d);
+        return bfail(b, PS_ERR_CUDA, "block table: %s", cudaGetErrorString(e));
+    }
+    b->tables.push_back({vw, vh, (int)u.size(), d});
+    *index = (int)b->tables.size() - 1;
+    return PS_OK;
+}
+
+// The launches of a run of nlevels levels, with their tables.
+int batch_block_steps(ps_batch* b, int64_t nlevels, std::vector<BlockStep>* steps)
+{
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
+    std::vector<BlockGrid> gs;
+    for (const auto& I : b->inst) gs.push_back({I.nx, I.ny});
+    const BlockGrids g{gs.data(), (int)gs.size()};
+    if (nlevels <= 0) return PS_OK;
+    const BlockPlan plan = plan_block(kTilesFE, g, (int)std::min<int64_t>(nlevels, 1 << 20), 1,
+                                      kTileMaxT, sms);
+    const int rows = stream_rows(g, sms);
+    BlockStep s{};
+    int T = 0;
+    for (int64_t done = 0; done < nlevels; done += T) {
+        const int t = plan_next(plan, nlevels - done, 1);
+        if (t != T) {
+            T = t;
+            s.T = T;
+            s.stream = plan.stream && T == kStreamT;
+            double us;
+            if (!s.stream) s.tile = best_tile(kTilesFE, T, g, sms, &us);
+            const int vw = s.stream ? kStreamW : tile_vw(s.tile, T);
+            const int vh = s.stream ? rows : tile_vh(s.tile, T);
+            if (int rc = batch_table(b, vw, vh, &s.table)) return rc;
+        }
+        steps->push_back(s);
+    }
+    return PS_OK;
+}
+
+int batch_block_upload(ps_batch* b)
+{
+    if (b->binst_current) return PS_OK;
+    std::vector<BlockInst> d;
+    for (const auto& I : b->inst)
+        d.push_back({{I.base[0], I.base[1]}, make_params_g(b->eq, I.globals).d[0], I.nx, I.ny});
+    PSB_CUDA(b, cudaMemcpyAsync(b->d_binst, d.data(), d.size() * sizeof(BlockInst),
+                                cudaMemcpyHostToDevice, b->stream));
+    PSB_CUDA(b, cudaStreamSynchronize(b->stream));
+    b->binst_current = true;
+    return PS_OK;
+}
+
+template <int C, int R, int MAXW>
+void launch_tile_batch(ps_batch* b, const BlockStep& s, const ps_batch::Table& t, int par)
+{
+    auto k = heat_block_tile_batch<C, R, MAXW>;
+    const size_t smem = tile_smem<C>(s.tile.nw);
+    if (smem > 48 * 1024) allow_big_smem(k);
+    launch_after(k, t.n, 32 * s.tile.nw, smem, b->stream, (const BlockInst*)b->d_binst,
+                 (const int2*)t.d, par, s.T, t.vw, t.vh);
+}
+
+int batch_block_enqueue(ps_batch* b, const std::vector<BlockStep>& steps)
+{
+    int par = b->cur;
+    for (const BlockStep& s : steps) {
+        const ps_batch::Table& t = b->tables[s.table];
+        if (s.stream)
+            launch_after(heat_block_stream_batch, t.n, 32, 0, b->stream, (const BlockInst*)b->d_binst,
+                         (const int2*)t.d, par, t.vh);
+        else if (s.tile.C == 4) launch_tile_batch<4, 6, 16>(b, s, t, par);
+        else if (s.tile.R == 8) launch_tile_batch<2, 8, 20>(b, s, t, par);
+        else launch_tile_batch<2, 4, 24>(b, s, t, par);
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return bfail(b, PS_ERR_CUDA, "batched launch: %s", cudaGetErrorString(e));
+        par ^= 1;
+    }
+    return PS_OK;
+}
+
 // Enqueue a whole run of nlevels levels, starting from parity b->cur.
 int batch_enqueue(ps_batch* b, int64_t nlevels, HalfFn half, int64_t* nlaunch)
 {
-    // (the register heat streams' descriptor copies come first in their
-    // shared memory)
-    const size_t ssm = batch_seam_smem(b),
-                 gsm = batch_stream_smem(b) + (b->fast ? kFastWarps * kDescBytes : 0);
-    const dim3 fgrid((b->nunits + kFastWarps - 1) / kFastWarps);
+    const size_t ssm = batch_seam_smem(b), gsm = batch_stream_smem(b);
     const size_t fe = (size_t)b->nv;
     int par = b->cur;
     int64_t done = 0, n = 0;
@@ -1914,7 +1983,7 @@ int batch_enqueue(ps_batch* b, int64_t nlevels, HalfFn half, int64_t* nlaunch)
                                                 cudaMemcpyDeviceToDevice, b->stream));
             }
         }
-        half(b, par, H, done, ssm, gsm, fgrid);
+        half(b, par, H, done, ssm, gsm);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return bfail(b, PS_ERR_CUDA, "batched launch: %s", cudaGetErrorString(e));
         n += 4;
@@ -2018,13 +2087,16 @@ int ps_batch_create(ps_batch** out, int device, int equation, int count, const i
         I.yface_n = yn;
         cudaError_t e = cudaMalloc(&I.base[0], f * its * sizeof(double));
         if (e == cudaSuccess) e = cudaMalloc(&I.base[1], f * its * sizeof(double));
-        if (e == cudaSuccess && xn) e = cudaMalloc(&I.xface, xn * sizeof(double));
-        if (e == cudaSuccess && yn) e = cudaMalloc(&I.yface, yn * sizeof(double));
+        // (the overlapped blocks keep no faces)
+        if (e == cudaSuccess && xn && !b->fast) e = cudaMalloc(&I.xface, xn * sizeof(double));
+        if (e == cudaSuccess && yn && !b->fast) e = cudaMalloc(&I.yface, yn * sizeof(double));
         if (e != cudaSuccess) rc = bfail(b, PS_ERR_NOMEM, "instance buffers: %s", cudaGetErrorString(e));
     }
     if (rc == PS_OK) {
         b->nunits = (int)units.size();
         cudaError_t e = cudaMalloc(&b->d_desc, 4 * b->inst.size() * sizeof(SweptArgs));
+        if (e == cudaSuccess && b->fast)
+            e = cudaMalloc(&b->d_binst, b->inst.size() * sizeof(BlockInst));
         if (e == cudaSuccess) e = cudaMalloc(&b->d_units, units.size() * sizeof(int2));
         if (e == cudaSuccess)
             e = cudaMemcpy(b->d_units, units.data(), units.size() * sizeof(int2), cudaMemcpyHostToDevice);
@@ -2056,6 +2128,8 @@ int ps_batch_destroy(ps_batch* b)
         if (I.xface) cudaFree(I.xface);
         if (I.yface) cudaFree(I.yface);
     }
+    if (b->d_binst) cudaFree(b->d_binst);
+    for (auto& t : b->tables) cudaFree(t.d);
     if (b->d_desc) cudaFree(b->d_desc);
     if (b->d_units) cudaFree(b->d_units);
     if (b->side) {
@@ -2080,6 +2154,7 @@ int ps_batch_set_global(ps_batch* b, int index, const char* name, const void* va
     for (int i = 0; i < (int)b->inst.size(); ++i)
         if (index == -1 || index == i) b->inst[i].globals[name] = v;
     batch_free_graph(b);  // constants live in the captured descriptors
+    b->binst_current = false;
     return PS_OK;
 }
 
@@ -2112,22 +2187,37 @@ int ps_batch_run(ps_batch* b, int64_t nlevels, int use_graph)
     PrepFn prep;
     batch_pick((b->eq == PS_EQ_EULER && !b->faces) ? PS_EQ_EULER_CELL : b->eq, b->ops, b->its,
                b->chunk, &half, &prep);
-    const int64_t nhalf = (nlevels + b->H - 1) / b->H;
+    int64_t nsteps = (nlevels + b->H - 1) / b->H;  // half-cycles, or block launches
+    std::vector<BlockStep> steps;
+    const bool rebuild = !use_graph || !b->gexec || b->graph_levels != nlevels || b->graph_cur != b->cur;
+    if (b->fast && rebuild) {
+        int rc = batch_block_steps(b, nlevels, &steps);
+        if (rc) return rc;
+        nsteps = (int64_t)steps.size();
+    } else if (b->fast) {
+        nsteps = b->graph_launches;
+    }
+    auto upload = [&]() -> int { return b->fast ? batch_block_upload(b) : batch_upload(b); };
+    auto enqueue = [&](int64_t* n) -> int {
+        if (!b->fast) return batch_enqueue(b, nlevels, half, n);
+        *n = (int64_t)steps.size();
+        return batch_block_enqueue(b, steps);
+    };
     if (!use_graph) {
-        int rc = batch_upload(b);
+        int rc = upload();
         if (rc) return rc;
         int64_t n = 0;
-        rc = batch_enqueue(b, nlevels, half, &n);
+        rc = enqueue(&n);
         if (rc) return rc;
         b->launches += n;
     } else {
-        if (!b->gexec || b->graph_levels != nlevels || b->graph_cur != b->cur) {
+        if (rebuild) {
             batch_free_graph(b);
-            int rc = batch_upload(b);
+            int rc = upload();
             if (rc) return rc;
             PSB_CUDA(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
             int64_t n = 0;
-            rc = batch_enqueue(b, nlevels, half, &n);
+            rc = enqueue(&n);
             cudaGraph_t g = nullptr;
             cudaError_t e = cudaStreamEndCapture(b->stream, &g);
             if (rc) {
@@ -2140,14 +2230,14 @@ int ps_batch_run(ps_batch* b, int64_t nlevels, int use_graph)
             b->graph_levels = nlevels;
             b->graph_cur = b->cur;
             b->graph_launches = n;
-        } else if (!batch_desc_current(b)) {
+        } else if (!b->fast && !batch_desc_current(b)) {
             int rc = batch_upload(b);  // new level counters for the same graph
             if (rc) return rc;
         }
         PSB_CUDA(b, cudaGraphLaunch(b->gexec, b->stream));
         b->launches += b->graph_launches;
     }
-    b->cur ^= (int)(nhalf & 1);
+    b->cur ^= (int)(nsteps & 1);
     for (auto& I : b->inst) I.level += nlevels;
     return PS_OK;
 }

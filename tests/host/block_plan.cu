@@ -18,7 +18,9 @@ int check(const TileShape (&shapes)[N], int step, int sms)
                 for (int maxT : {step, 3, 8, 16}) {
                     const int nl = n - n % step;
                     if (nl < step || maxT < step) continue;
-                    const BlockPlan p = plan_block(shapes, nx, ny, nl, step, maxT, sms);
+                    const BlockGrid one{nx, ny};
+                    const BlockGrids g{&one, 1};
+                    const BlockPlan p = plan_block(shapes, g, nl, step, maxT, sms);
                     if (p.T < step || p.T % step || p.T > kTileMaxT || (p.T > maxT && maxT % step == 0) ||
                         (p.stream && (p.T != kStreamT || maxT < kStreamT))) {
                         printf("plan %dx%d n %d maxT %d: T %d\n", nx, ny, nl, maxT, p.T);
@@ -26,7 +28,7 @@ int check(const TileShape (&shapes)[N], int step, int sms)
                     }
                     for (int T = step; T <= p.T; T += step) {
                         double us;
-                        const TileShape t = best_tile(shapes, T, nx, ny, sms, &us);
+                        const TileShape t = best_tile(shapes, T, g, sms, &us);
                         const int halo = (32 * t.C - tile_vw(t, T)) / 2;
                         if (tile_vh(t, T) < 2 || tile_vw(t, T) < 8 || halo < T || halo % t.C ||
                             t.nw > t.maxw || !(us < 1e300)) {
@@ -34,7 +36,7 @@ int check(const TileShape (&shapes)[N], int step, int sms)
                             return 1;
                         }
                     }
-                    const int rows = stream_rows(nx, ny, sms);
+                    const int rows = stream_rows(g, sms);
                     if (rows < 1 || rows > nx) {
                         printf("strip rows %d of %d\n", rows, nx);
                         return 1;

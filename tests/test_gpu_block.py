@@ -109,3 +109,23 @@ def test_configured_levels_bound_a_launch(h):
     (u,), _ = _solve(ic, g, 1, 16, nl, h=h)
     _, ref, _ = oracle.standard("heat", ic, g, 1, nl, frames=False)
     assert np.array_equal(u, ref)
+
+
+@pytest.mark.parametrize("sizes,runs", [
+    ([(32, 32), (128, 480), (64, 160)], (5, 17)),          # tiles
+    ([(2048, 2048), (64, 96), (32, 1056)], (20, 3)),       # streams, then tiles
+])
+@pytest.mark.parametrize("graph", [True, False])
+def test_batched_blocks(sizes, runs, graph):
+    from pysweep_b200 import Batch, plugin_constants
+    ics = [_ic(nx, ny) for nx, ny in sizes]
+    with Batch("heat", sizes, its=1, blocksize=16) as b:
+        for i, (nx, _) in enumerate(sizes):
+            b.set_constants(i, plugin_constants("heat", _globals(nx)))
+            b.set_state(i, ics[i])
+        for n in runs:
+            b.run(n, graph=graph)
+        got = [b.get_state(i) for i in range(len(sizes))]
+    for u, ic in zip(got, ics):
+        (ref,), _ = _solve(ic, _globals(ic.shape[1]), 1, 16, sum(runs), mode="standard", threads=256)
+        assert np.array_equal(u, ref)
