@@ -18,7 +18,7 @@
 #include "seam_fast.cuh"
 #include "heat_block.cuh"
 #include "standard_fast.cuh"
-#include "euler_faces.cuh"
+#include "euler_march.cuh"
 #include "batch.cuh"
 #include "hook.cuh"
 
@@ -704,6 +704,66 @@ int run_block(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
     return PS_OK;
 }
 
+// Euler level by level (euler_march.cuh), for either decomposition: its levels
+// are bound by arithmetic, not by memory, so a cell evaluated twice costs more
+// than a level kept on chip saves (prisms of blocksize 16 at 4096²: 6.3 G cell
+// stages/s, at 1120² 5.1; level by level 18.7 and 16.0).  The two base buffers
+// hold four levels: each new one goes to the oldest slot.
+int run_march(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t frame_cap,
+              int frame_every, int kind)
+{
+    const size_t fe = field_elems(s);
+    const int every = frame_every > 0 ? frame_every : 1;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
+    const EqParams prm = make_params(s);
+    const BlockGrid grid{s->nx, s->ny};
+    MarchArgs a;
+    memset(&a, 0, sizeof a);
+    a.nx = s->nx;
+    a.ny = s->ny;
+    a.ncs = (s->ny + kMarchW - 1) / kMarchW;
+    a.hs = march_rows(BlockGrids{&grid, 1}, sms);
+    a.dtdx = prm.d[0];
+    a.dtdy = prm.d[1];
+    a.gamma = prm.d[2];
+    a.gm1 = prm.d[3];
+    const int units = a.ncs * ((s->nx + a.hs - 1) / a.hs);
+    double* slot[4];  // [base][older, newer]
+    for (int q = 0; q < 4; ++q) slot[q] = at(s, s->base[q / 2], (size_t)(q % 2) * fe);
+    int older = 2 * s->cur, newest = older + 1;  // slots of levels L-2 and L-1
+    for (int64_t L = 1; L <= nlevels; ++L) {
+        const int next = newest % 2 ? (newest + 1) % 4 : newest + 1;
+        double* fr = nullptr;
+        if (frames && L % 2 == 0 && (L / 2) % every == 0) {
+            const int64_t k = (L / 2) / every - 1;
+            if (k < frame_cap) fr = at(s, frames, (size_t)k * fe);
+        }
+        const bool direct = reinterpret_cast<uintptr_t>(fr) % 16 == 0;
+        a.cur = slot[newest];
+        a.prev = slot[older];
+        a.out = slot[next];
+        a.frame = direct ? fr : nullptr;
+        a.gts = gts0 + (int)(L - 1);
+        int rc = timed_launch(s, kind, (double)s->nx * s->ny,
+                              [&] { launch_after(euler_march, units, 32, 0, s->stream, a); });
+        if (rc) return rc;
+        if (fr && !direct)
+            PS_CUDA(s, cudaMemcpyAsync(fr, a.out, nbytes(s, fe), cudaMemcpyDeviceToDevice, s->stream));
+        older = newest;
+        newest = next;
+    }
+    s->cur = newest / 2;
+    if (newest % 2 == 0) {
+        // an odd count: the newest level moves up beside the one before it
+        PS_CUDA(s, cudaMemcpyAsync(slot[newest + 1], slot[newest], nbytes(s, fe),
+                                   cudaMemcpyDeviceToDevice, s->stream));
+        PS_CUDA(s, cudaMemcpyAsync(slot[newest], slot[older], nbytes(s, fe), cudaMemcpyDeviceToDevice,
+                                   s->stream));
+    }
+    return PS_OK;
+}
+
 int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t frame_cap,
               int frame_every)
 {
@@ -820,6 +880,8 @@ int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
         if (maxT >= 2 && aligned32(frames))
             return run_block<double, true>(s, nlevels, gts0, frames, frame_cap, frame_every, maxT);
     }
+    if (s->eq == PS_EQ_EULER && s->threads != 256 && march_constants(make_params(s)))
+        return run_march(s, nlevels, gts0, frames, frame_cap, frame_every, 5);
     int rc = ensure_swept_buffers(s);
     if (rc) return rc;
     if (!s->side) {
@@ -922,6 +984,9 @@ int run_standard(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_
 {
     StdLaunch K = s->hook ? nullptr : pick_standard(s->eq, s->ops);
     if (!K && !s->hook) return fail(s, PS_ERR_UNSUPPORTED, "no standard kernel for equation %d", s->eq);
+    // (threads = 256 keeps the per-cell kernel)
+    if (s->eq == PS_EQ_EULER && s->threads != 256 && march_constants(make_params(s)))
+        return run_march(s, nlevels, gts0, frames, frame_cap, frame_every, 4);
     const size_t fe = field_elems(s);
     for (int i = 0; i < 3; ++i)
         if (!s->ring[i]) PS_CUDA(s, cudaMalloc(&s->ring[i], nbytes(s, fe)));
@@ -938,9 +1003,6 @@ int run_standard(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_
     // streaming heat kernel (64-column strips); threads = 256 keeps the generic one
     const bool fast = s->eq == PS_EQ_HEAT && s->ny % 64 == 0 && s->threads != 256;
     const bool f32 = s->dtype == PS_DTYPE_F32;
-    // Euler: faces shared between cells (threads = 256 keeps the per-cell kernel)
-    const bool euler_faces = s->eq == PS_EQ_EULER && s->threads != 256;
-    if (euler_faces) allow_big_smem(euler_standard_faces);
     if (f32 && !(fast && prm.i[0]))
         return fail(s, PS_ERR_UNSUPPORTED,
                     "float32 fields: heat with forward Euler and ny a multiple of 64 only");
@@ -981,10 +1043,6 @@ int run_standard(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_
                      else
                          heat_standard_fast<true><<<grid, 256, 0, s->stream>>>(
                              s->ring[c], s->ring[p], s->ring[n], fr, s->nx, s->ny, gts, prm.d[0]);
-                 } else if (euler_faces) {
-                     const dim3 grid((s->ny + kEuTC - 1) / kEuTC, (s->nx + kEuTR - 1) / kEuTR);
-                     euler_standard_faces<<<grid, 256, kEuStdSmem, s->stream>>>(
-                         s->ring[c], s->ring[p], s->ring[n], fr, s->nx, s->ny, gts, prm);
                  } else {
                      K(s->ring[c], s->ring[p], s->ring[n], fr, s->nx, s->ny, s->nv, gts, prm,
                        s->stream);
