@@ -471,22 +471,29 @@ struct BlockGrids {
     }
 };
 
+// A tile's work relative to plain heat's: FP64 pipe time of a level, bytes of a
+// tile, latency of a level.
+struct TileCost {
+    double level = 1.0, bytes = 1.0, latency = 1.0;
+};
+
 // Estimated microseconds of one launch of T levels in tiles of shape t, or 0
 // where no cell of the tile stays exact.  Fitted to launches of 160² to 8192²
 // (within 15%): a level of one tile takes its FP64 operations at the pipe's
 // rate (16 cycles per warp and cell) and, with few warps on the SM, the latency
 // of the exchange; loading and storing cost 0.03 us per KB of the tiles on an
 // SM, hidden behind other tiles where the SM holds more than one.
-inline double tile_us(const TileShape& t, int T, const BlockGrids& g, int sms)
+inline double tile_us(const TileShape& t, int T, const BlockGrids& g, int sms,
+                      const TileCost& c = TileCost{})
 {
     const int vw = tile_vw(t, T), vh = tile_vh(t, T);
     if (vw < 8 || vh < 2) return 0.0;
     const double n = (double)((g.blocks(vw, vh) + sms - 1) / sms);  // tiles of the busiest SM
     const int occ = t.maxw / t.nw;
     const double k = std::min(n, (double)occ), rounds = std::max(1.0, n / occ);
-    const double level = 4.0 * t.nw * t.R * t.C / 1965.0 * 1.04;
-    const double kb = k * t.nw * t.R * t.C * 32 * 8 / 1024.0 * 0.03;
-    const double lat = k * t.nw <= 12 ? 0.08 : 0.03;
+    const double level = 4.0 * t.nw * t.R * t.C / 1965.0 * 1.04 * c.level;
+    const double kb = k * t.nw * t.R * t.C * 32 * 8 / 1024.0 * 0.03 * c.bytes;
+    const double lat = (k * t.nw <= 12 ? 0.08 : 0.03) * c.latency;
     return 1.0 + n * T * level + (occ == 1 ? rounds : 1.0) * kb + (n - k) * 0.4 + lat * T * rounds;
 }
 
@@ -506,16 +513,32 @@ inline int stream_rows(const BlockGrids& g, int sms)
 // The cheapest tile for one launch of T levels.
 template <int NSHAPE>
 inline TileShape best_tile(const TileShape (&shapes)[NSHAPE], int T, const BlockGrids& g, int sms,
-                           double* us)
+                           double* us, const TileCost& cost = TileCost{})
 {
     TileShape best = shapes[0];
     *us = 1e300;
     for (const TileShape& t : shapes) {
-        const double one = tile_us(t, T, g, sms);
+        const double one = tile_us(t, T, g, sms, cost);
         if (one > 0 && one < *us) {
             *us = one;
             best = t;
         }
+    }
+    return best;
+}
+
+// The cheapest way to run nlevels levels in tiles.
+template <int NSHAPE>
+inline BlockPlan plan_tiles(const TileShape (&shapes)[NSHAPE], const BlockGrids& g, int nlevels,
+                            int step, int maxT, int sms, const TileCost& cost = TileCost{})
+{
+    BlockPlan best{false, step, 1e300};
+    for (int T = step; T <= std::min(maxT, kTileMaxT); T += step) {
+        const int k = (nlevels + T - 1) / T;
+        const int Tk = ((nlevels + k - 1) / k + step - 1) / step * step;  // even shares
+        double one;
+        best_tile(shapes, Tk, g, sms, &one, cost);
+        if (k * one < best.us) best = BlockPlan{false, Tk, k * one};
     }
     return best;
 }
@@ -528,14 +551,7 @@ template <int NSHAPE>
 inline BlockPlan plan_block(const TileShape (&shapes)[NSHAPE], const BlockGrids& g, int nlevels,
                             int step, int maxT, int sms)
 {
-    BlockPlan best{false, step, 1e300};
-    for (int T = step; T <= std::min(maxT, kTileMaxT); T += step) {
-        const int k = (nlevels + T - 1) / T;
-        const int Tk = ((nlevels + k - 1) / k + step - 1) / step * step;  // even shares
-        double one;
-        best_tile(shapes, Tk, g, sms, &one);
-        if (k * one < best.us) best = BlockPlan{false, Tk, k * one};
-    }
+    BlockPlan best = plan_tiles(shapes, g, nlevels, step, maxT, sms);
     if (nlevels >= kStreamT && maxT >= kStreamT) {
         const int rows = stream_rows(g, sms);
         // (strips of very wide grids, or of many, may fill more than one wave)
@@ -584,17 +600,18 @@ __device__ __forceinline__ void batch_block_args(const BlockInst* inst, int i, i
     a.cr = b.cr;
 }
 
+template <class S>
 __global__ void __launch_bounds__(32, 8)
     heat_block_stream_batch(const BlockInst* __restrict__ inst, const int2* __restrict__ units,
                             int par, int vh)
 {
-    __shared__ __align__(16) double ring[kBlockRing * 32 * kStreamC];
+    __shared__ __align__(16) S ring[kBlockRing * 32 * kStreamC];
     const int2 u = units[blockIdx.x];
     BlockArgs a;
     batch_block_args(inst, u.x, par, kStreamT, kStreamW, vh, a);
     grid_wait();
     grid_release();
-    block_stream_body<double, false>(a, u.y, ring);
+    block_stream_body<S, false>(a, u.y, ring);
 }
 
 template <int C, int R, int MAXW>

@@ -17,6 +17,8 @@
 #include "heat_fast.cuh"
 #include "seam_fast.cuh"
 #include "heat_block.cuh"
+#include "heatvar_block.cuh"
+#include "launch.cuh"
 #include "standard_fast.cuh"
 #include "euler_march.cuh"
 #include "batch.cuh"
@@ -114,24 +116,6 @@ namespace {
 
 const char* kVersion = "pysweep_b200 0.1.0 (sm_100a)";
 thread_local std::string g_create_error;  // message of the last failed ps_create
-
-// Opt a kernel into the large dynamic shared-memory carve-out, once per
-// (kernel, device).
-std::mutex g_attr_mu;
-std::map<std::pair<const void*, int>, bool> g_attr_done;
-
-template <class K>
-void allow_big_smem(K kernel)
-{
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const auto key = std::make_pair(reinterpret_cast<const void*>(kernel), dev);
-    std::lock_guard<std::mutex> lock(g_attr_mu);
-    if (!g_attr_done[key]) {
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        g_attr_done[key] = true;
-    }
-}
 
 int fail(ps_solver* s, int code, const char* fmt, ...)
 {
@@ -546,24 +530,6 @@ int hook_frame(ps_solver* s, int ns, int rows, int cols, int times)
 }
 
 // ------------------------------------------------- overlapped heat blocks ----
-// A kernel that may begin while the one before it in the stream ends (it waits
-// for it itself: grid_wait).
-template <class... A>
-void launch_after(void (*k)(A...), int grid, int nt, size_t smem, cudaStream_t st, A... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(nt);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k, args...);
-}
-
 template <class S, bool RK2, int C, int R, int MAXW>
 void launch_tile(const BlockArgs& a, int nw, cudaStream_t st)
 {
@@ -701,6 +667,71 @@ int run_block(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
                                        cudaMemcpyDeviceToDevice, s->stream));
     }
     if (done < nlevels && (rc = single())) return rc;
+    return PS_OK;
+}
+
+// The fields of a per-cell-courant solver can be copied 16 bytes at a time.
+bool var_aligned(const ps_solver* s)
+{
+    for (const double* f : s->field)
+        if (reinterpret_cast<uintptr_t>(f) % 16) return false;
+    return s->ny % 2 == 0;
+}
+
+// The per-cell-courant equations in overlapped tiles (heatvar_block.cuh).
+// Level L of the run has globalTimeStep gts0 + L - 1; the forward stores its old
+// level's Laplacian at index gts - 1 of field 1, the adjoint reads index LEN -
+// gts (ps_run has checked that they lie in it).  A frame ends its launch and is
+// copied from the state.
+template <int ROLE>
+int run_var(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t frame_cap,
+            int frame_every)
+{
+    const size_t fe = field_elems(s), plane = (size_t)s->nx * s->ny;
+    const int every = frame_every > 0 ? frame_every : 1;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
+    const EqParams prm = make_params(s);
+    const BlockGrid grid{s->nx, s->ny};
+    VarArgs a;
+    memset(&a, 0, sizeof a);
+    a.C = prm.f[0];
+    a.nx = s->nx;
+    a.ny = s->ny;
+    a.step = ROLE >= VAR_LAMBDA ? -(long long)plane : (long long)plane;
+    BlockPlan plan{};
+    if (nlevels > 0)
+        plan = plan_var<ROLE>(BlockGrids{&grid, 1}, (int)std::min<int64_t>(nlevels, 1 << 20), sms);
+    int rc;
+    for (int64_t done = 0; done < nlevels;) {
+        int T = plan_next(plan, nlevels - done, 1);
+        double* fr = nullptr;
+        for (int m = 1; frames && m <= T; ++m)
+            if ((done + m) % every == 0 && (done + m) / every - 1 < frame_cap) {
+                fr = at(s, frames, (size_t)((done + m) / every - 1) * fe);
+                T = m;
+            }
+        const int64_t gts = gts0 + done;  // of the launch's first level
+        a.in = s->base[s->cur];
+        a.out = s->base[1 - s->cur];
+        if (ROLE == VAR_RECOMPUTE) a.lap = prm.f[1] + (gts - 1) * plane;
+        if (ROLE >= VAR_LAMBDA) a.lap = prm.f[1] + (prm.i[3] - gts) * (int64_t)plane;
+        if (ROLE == VAR_MU) a.g = prm.f[2];
+        if (ROLE == VAR_LAMBDA) {
+            // the second variable, from one base to the other
+            a.g = s->base[1 - s->cur] + plane;
+            PS_CUDA(s, cudaMemcpyAsync(a.g, s->base[s->cur] + plane, plane * sizeof(double),
+                                       cudaMemcpyDeviceToDevice, s->stream));
+        }
+        if ((rc = timed_launch(s, 5, (double)plane * T,
+                               [&] { launch_var<ROLE>(a, T, sms, s->stream); })))
+            return rc;
+        s->cur = 1 - s->cur;
+        done += T;
+        if (fr)
+            PS_CUDA(s, cudaMemcpyAsync(fr, s->base[s->cur], nbytes(s, fe), cudaMemcpyDeviceToDevice,
+                                       s->stream));
+    }
     return PS_OK;
 }
 
@@ -882,6 +913,16 @@ int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
     }
     if (s->eq == PS_EQ_EULER && s->threads != 256 && march_constants(make_params(s)))
         return run_march(s, nlevels, gts0, frames, frame_cap, frame_every, 5);
+    if (s->threads != 256 && var_aligned(s)) {
+        if (s->eq == PS_EQ_HEATVAR && !s->field[1])
+            return run_var<VAR_FORWARD>(s, nlevels, gts0, frames, frame_cap, frame_every);
+        if (s->eq == PS_EQ_HEATVAR)
+            return run_var<VAR_RECOMPUTE>(s, nlevels, gts0, frames, frame_cap, frame_every);
+        if (s->eq == PS_EQ_HEATVAR_ADJ)
+            return run_var<VAR_LAMBDA>(s, nlevels, gts0, frames, frame_cap, frame_every);
+        if (s->eq == PS_EQ_HEATVAR_ADJMU)
+            return run_var<VAR_MU>(s, nlevels, gts0, frames, frame_cap, frame_every);
+    }
     int rc = ensure_swept_buffers(s);
     if (rc) return rc;
     if (!s->side) {
@@ -2011,7 +2052,7 @@ int batch_block_enqueue(ps_batch* b, const std::vector<BlockStep>& steps)
     for (const BlockStep& s : steps) {
         const ps_batch::Table& t = b->tables[s.table];
         if (s.stream)
-            launch_after(heat_block_stream_batch, t.n, 32, 0, b->stream, (const BlockInst*)b->d_binst,
+            launch_after(heat_block_stream_batch<double>, t.n, 32, 0, b->stream, (const BlockInst*)b->d_binst,
                          (const int2*)t.d, par, t.vh);
         else if (s.tile.C == 4) launch_tile_batch<4, 6, 16>(b, s, t, par);
         else if (s.tile.R == 8) launch_tile_batch<2, 8, 20>(b, s, t, par);
