@@ -600,8 +600,8 @@ int run_block(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
         double* fr = frame_of(done + 1);
         const int gts = gts0 + (int)done;
         if (int e = timed_launch(s, 4, (double)s->nx * s->ny, [&] {
-                launch_standard<Heat>(newest(b), s->base[b], newest(1 - b), fr, s->nx, s->ny, 1,
-                                      gts, prm, s->stream);
+                launch_standard<Heat>(newest(b), s->base[b], newest(1 - b), fr, s->nx, s->ny, 1, gts,
+                                      prm, s->stream);
             }))
             return e;
         PS_CUDA(s, cudaMemcpyAsync(s->base[1 - b], newest(b), nbytes(s, fe),
@@ -735,16 +735,56 @@ int run_var(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t fra
     return PS_OK;
 }
 
+// Level by level in the base buffers: they hold 2 its levels, and each new one
+// goes to the oldest slot, so no field is copied but after an odd count of
+// two-stage levels.  launch(cur, prev, out, frame, gts) queues one level; prev is
+// the level before cur (two base levels).  A frame that 16-byte stores cannot
+// reach is copied from its level.
+template <class F>
+int run_levels(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t frame_cap,
+               int frame_every, int kind, F&& launch)
+{
+    const size_t fe = field_elems(s);
+    const int its = s->its, every = frame_every > 0 ? frame_every : 1;
+    double* slot[4];  // [base][its: older, newer]
+    for (int q = 0; q < 2 * its; ++q) slot[q] = at(s, s->base[q / its], (size_t)(q % its) * fe);
+    int older = its * s->cur, newest = older + its - 1;  // slots of levels L-2 and L-1
+    for (int64_t L = 1; L <= nlevels; ++L) {
+        const int next = (newest + 1) % (2 * its);
+        double* fr = nullptr;
+        if (frames && L % its == 0 && (L / its) % every == 0) {
+            const int64_t k = (L / its) / every - 1;
+            if (k < frame_cap) fr = at(s, frames, (size_t)k * fe);
+        }
+        const bool direct = reinterpret_cast<uintptr_t>(fr) % 16 == 0;
+        int rc = timed_launch(s, kind, (double)s->nx * s->ny, [&] {
+            launch(slot[newest], slot[older], slot[next], direct ? fr : nullptr, gts0 + (int)(L - 1));
+        });
+        if (rc) return rc;
+        if (fr && !direct)
+            PS_CUDA(s, cudaMemcpyAsync(fr, slot[next], nbytes(s, fe), cudaMemcpyDeviceToDevice,
+                                       s->stream));
+        older = newest;
+        newest = next;
+    }
+    s->cur = newest / its;
+    if (its == 2 && newest % 2 == 0) {
+        // an odd count: the newest level moves up beside the one before it
+        PS_CUDA(s, cudaMemcpyAsync(slot[newest + 1], slot[newest], nbytes(s, fe),
+                                   cudaMemcpyDeviceToDevice, s->stream));
+        PS_CUDA(s, cudaMemcpyAsync(slot[newest], slot[older], nbytes(s, fe), cudaMemcpyDeviceToDevice,
+                                   s->stream));
+    }
+    return PS_OK;
+}
+
 // Euler level by level (euler_march.cuh), for either decomposition: its levels
 // are bound by arithmetic, not by memory, so a cell evaluated twice costs more
 // than a level kept on chip saves (prisms of blocksize 16 at 4096²: 6.3 G cell
-// stages/s, at 1120² 5.1; level by level 18.7 and 16.0).  The two base buffers
-// hold four levels: each new one goes to the oldest slot.
+// stages/s, at 1120² 5.1; level by level 18.7 and 16.0).
 int run_march(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t frame_cap,
               int frame_every, int kind)
 {
-    const size_t fe = field_elems(s);
-    const int every = frame_every > 0 ? frame_every : 1;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
     const EqParams prm = make_params(s);
@@ -760,39 +800,33 @@ int run_march(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
     a.gamma = prm.d[2];
     a.gm1 = prm.d[3];
     const int units = a.ncs * ((s->nx + a.hs - 1) / a.hs);
-    double* slot[4];  // [base][older, newer]
-    for (int q = 0; q < 4; ++q) slot[q] = at(s, s->base[q / 2], (size_t)(q % 2) * fe);
-    int older = 2 * s->cur, newest = older + 1;  // slots of levels L-2 and L-1
-    for (int64_t L = 1; L <= nlevels; ++L) {
-        const int next = newest % 2 ? (newest + 1) % 4 : newest + 1;
-        double* fr = nullptr;
-        if (frames && L % 2 == 0 && (L / 2) % every == 0) {
-            const int64_t k = (L / 2) / every - 1;
-            if (k < frame_cap) fr = at(s, frames, (size_t)k * fe);
-        }
-        const bool direct = reinterpret_cast<uintptr_t>(fr) % 16 == 0;
-        a.cur = slot[newest];
-        a.prev = slot[older];
-        a.out = slot[next];
-        a.frame = direct ? fr : nullptr;
-        a.gts = gts0 + (int)(L - 1);
-        int rc = timed_launch(s, kind, (double)s->nx * s->ny,
-                              [&] { launch_after(euler_march, units, 32, 0, s->stream, a); });
-        if (rc) return rc;
-        if (fr && !direct)
-            PS_CUDA(s, cudaMemcpyAsync(fr, a.out, nbytes(s, fe), cudaMemcpyDeviceToDevice, s->stream));
-        older = newest;
-        newest = next;
-    }
-    s->cur = newest / 2;
-    if (newest % 2 == 0) {
-        // an odd count: the newest level moves up beside the one before it
-        PS_CUDA(s, cudaMemcpyAsync(slot[newest + 1], slot[newest], nbytes(s, fe),
-                                   cudaMemcpyDeviceToDevice, s->stream));
-        PS_CUDA(s, cudaMemcpyAsync(slot[newest], slot[older], nbytes(s, fe), cudaMemcpyDeviceToDevice,
-                                   s->stream));
-    }
-    return PS_OK;
+    return run_levels(s, nlevels, gts0, frames, frame_cap, frame_every, kind,
+                      [&](const double* cur, const double* prev, double* out, double* fr, int gts) {
+                          a.cur = cur;
+                          a.prev = prev;
+                          a.out = out;
+                          a.frame = fr;
+                          a.gts = gts;
+                          launch_after(euler_march, units, 32, 0, s->stream, a);
+                      });
+}
+
+template <bool RK2, class T>
+int run_heat_standard(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t frame_cap,
+                      int frame_every)
+{
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
+    const double cr = make_params(s).d[0];
+    const int rows = standard_rows(s->nx, s->ny, sms);
+    const int units = (s->ny + 63) / 64 * ((s->nx + rows - 1) / rows);
+    return run_levels(s, nlevels, gts0, frames, frame_cap, frame_every, 4,
+                      [&](const double* cur, const double* prev, double* out, double* fr, int gts) {
+                          launch_after(rows == 4 ? heat_standard<RK2, 4, T> : heat_standard<RK2, 8, T>,
+                                       (units + kStdWarps - 1) / kStdWarps, 32 * kStdWarps, 0,
+                                       s->stream, (const T*)cur, (const T*)prev, (T*)out, (T*)fr,
+                                       s->nx, s->ny, gts, cr);
+                      });
 }
 
 int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t frame_cap,
@@ -1025,9 +1059,23 @@ int run_standard(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_
 {
     StdLaunch K = s->hook ? nullptr : pick_standard(s->eq, s->ops);
     if (!K && !s->hook) return fail(s, PS_ERR_UNSUPPORTED, "no standard kernel for equation %d", s->eq);
-    // (threads = 256 keeps the per-cell kernel)
+    // (threads = 256 keeps the per-cell kernels)
     if (s->eq == PS_EQ_EULER && s->threads != 256 && march_constants(make_params(s)))
         return run_march(s, nlevels, gts0, frames, frame_cap, frame_every, 4);
+    if (s->eq == PS_EQ_HEAT && s->threads != 256) {
+        const bool fwd = make_params(s).i[0] != 0;
+        if (s->dtype == PS_DTYPE_F32) {
+            if (fwd && s->ny % 64 == 0)
+                return run_heat_standard<false, float>(s, nlevels, gts0, frames, frame_cap, frame_every);
+        } else if (fwd) {
+            return run_heat_standard<false, double>(s, nlevels, gts0, frames, frame_cap, frame_every);
+        } else if (s->its == 2) {
+            return run_heat_standard<true, double>(s, nlevels, gts0, frames, frame_cap, frame_every);
+        }
+    }
+    if (s->dtype == PS_DTYPE_F32)
+        return fail(s, PS_ERR_UNSUPPORTED,
+                    "float32 fields: heat with forward Euler and ny a multiple of 64 only");
     const size_t fe = field_elems(s);
     for (int i = 0; i < 3; ++i)
         if (!s->ring[i]) PS_CUDA(s, cudaMalloc(&s->ring[i], nbytes(s, fe)));
@@ -1041,12 +1089,6 @@ int run_standard(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_
                                nbytes(s, fe), cudaMemcpyDeviceToDevice, s->stream));
     const EqParams prm = make_params(s);
     const int every = frame_every > 0 ? frame_every : 1;
-    // streaming heat kernel (64-column strips); threads = 256 keeps the generic one
-    const bool fast = s->eq == PS_EQ_HEAT && s->ny % 64 == 0 && s->threads != 256;
-    const bool f32 = s->dtype == PS_DTYPE_F32;
-    if (f32 && !(fast && prm.i[0]))
-        return fail(s, PS_ERR_UNSUPPORTED,
-                    "float32 fields: heat with forward Euler and ny a multiple of 64 only");
     int rc;
     if (s->hook) {
         // the hook's standard tile: kHookStdTR x kHookStdTC cells and an
@@ -1072,18 +1114,6 @@ int run_standard(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_
                      hook_launch(s, s->hook->standard, (s->ny + kHookStdTC - 1) / kHookStdTC,
                                  (s->nx + kHookStdTR - 1) / kHookStdTR, kHookStdNT,
                                  3 * sizeof(double) * s->nv * tr * tc, s->stream, args);
-                 } else if (fast) {
-                     const dim3 grid((s->ny / 64 + 7) / 8, (s->nx + kStdRows - 1) / kStdRows);
-                     if (f32)
-                         heat_standard_fast<false, float><<<grid, 256, 0, s->stream>>>(
-                             (const float*)s->ring[c], (const float*)s->ring[p], (float*)s->ring[n],
-                             (float*)fr, s->nx, s->ny, gts, prm.d[0]);
-                     else if (prm.i[0])
-                         heat_standard_fast<false><<<grid, 256, 0, s->stream>>>(
-                             s->ring[c], s->ring[p], s->ring[n], fr, s->nx, s->ny, gts, prm.d[0]);
-                     else
-                         heat_standard_fast<true><<<grid, 256, 0, s->stream>>>(
-                             s->ring[c], s->ring[p], s->ring[n], fr, s->nx, s->ny, gts, prm.d[0]);
                  } else {
                      K(s->ring[c], s->ring[p], s->ring[n], fr, s->nx, s->ny, s->nv, gts, prm,
                        s->stream);
