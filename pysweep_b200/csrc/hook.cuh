@@ -33,8 +33,39 @@ constexpr const char* kHookNs[3] = {"psh_stream", "psh_seam", "psh_std"};
 enum HookFw { FW_VARS, FW_TIMES, FW_MPSS, FW_MOSS, FW_NV, FW_OPS, FW_ITS, FW_SX, FW_SY, FW_COUNT };
 constexpr const char* kHookFw[FW_COUNT] = {"VARS", "TIMES", "MPSS", "MOSS", "NV",
                                            "OPS",  "ITS",   "SX",   "SY"};
-// standard-step tile of the hook kernels (hook_kernels.cuh)
-constexpr int kHookStdTR = 16, kHookStdTC = 32, kHookStdNT = 256;
+// block tiles of the hook kernels (hook_kernels.cuh): columns of level 1, most
+// threads, most levels per launch.  Several levels run 512 threads (a step's
+// loads may not pass the store of the step before it, so warps have to cover
+// its latency; heat at 1024², us per level with 256 / 512 / 1024: 5.2, 4.6, 6.6),
+// one level 256 (8.5, 10.5, 15.9).
+constexpr int kHookBlkW = 64, kHookBlkNT = 512, kHookBlkMaxT = 8;
+
+// Rows of level 1 and levels of a block, or rows 0 where no tile fits.  Slots
+// of levels -1 .. T; the deepest block whose last level keeps two thirds of the
+// first one's cells and whose tile leaves room for two CTAs per SM; one level
+// (any room) where a second does not fit.
+struct HookBlock {
+    int rows, T;
+};
+inline int hook_block_threads(int T) { return T > 1 ? kHookBlkNT : kHookBlkNT / 2; }
+inline size_t hook_block_smem(int nv, int ops, int rows, int T)
+{
+    return sizeof(double) * (T + 2) * nv * (rows + 2 * ops) * (kHookBlkW + 2 * ops);
+}
+inline HookBlock hook_block(int nv, int ops, int maxT)
+{
+    for (int rows : {32, 16})
+        for (int T = maxT < kHookBlkMaxT ? maxT : kHookBlkMaxT; T >= 2; --T) {
+            const int ih = rows - 2 * ops * (T - 1), iw = kHookBlkW - 2 * ops * (T - 1);
+            const size_t sm = hook_block_smem(nv, ops, rows, T);
+            if (ih > 0 && iw > 0 && 3 * ih * iw >= 2 * rows * kHookBlkW && sm <= 113 * 1024)
+                return HookBlock{rows, T};
+        }
+    for (int rows : {32, 16, 8, 4})
+        if (hook_block_smem(nv, ops, rows, 1) <= (rows > 8 ? 113 : 227) * 1024)
+            return HookBlock{rows, 1};
+    return HookBlock{0, 0};
+}
 
 // A user constant, in every namespace (ps_get_global hands out a pointer to
 // it; `name` comes first, as in the built-in constants' table).
@@ -48,12 +79,11 @@ struct HookModule {
     CUmodule mod = nullptr;
     CUfunction prism[2] = {nullptr, nullptr};  // chunk 32, 64
     CUfunction gap[2] = {nullptr, nullptr};
-    CUfunction ybridge = nullptr, octahedron = nullptr, standard = nullptr;
+    CUfunction ybridge = nullptr, octahedron = nullptr, block = nullptr;
     CUdeviceptr fw[3][FW_COUNT] = {};
     int fw_val[3][FW_COUNT];  // last values written (-1: never)
     std::map<std::string, HookConst> consts;
     int nv = 1, ops = 1, its = 1;
-    size_t std_smem = 0;
     HookModule()
     {
         for (auto& r : fw_val)
@@ -72,6 +102,7 @@ struct Driver {
     decltype(&cuFuncSetAttribute) funcSetAttribute = nullptr;
     decltype(&cuMemcpyHtoDAsync) memcpyHtoDAsync = nullptr;
     decltype(&cuLaunchKernel) launchKernel = nullptr;
+    decltype(&cuLaunchKernelEx) launchKernelEx = nullptr;
     decltype(&cuGetErrorString) getErrorString = nullptr;
     bool ok = false;
 };
@@ -93,6 +124,7 @@ inline Driver& drv()
                get("cuFuncSetAttribute", (void**)&d.funcSetAttribute) &&
                get("cuMemcpyHtoDAsync", (void**)&d.memcpyHtoDAsync) &&
                get("cuLaunchKernel", (void**)&d.launchKernel) &&
+               get("cuLaunchKernelEx", (void**)&d.launchKernelEx) &&
                get("cuGetErrorString", (void**)&d.getErrorString);
     });
     return d;
@@ -167,9 +199,9 @@ inline std::string hook_program(const std::string& src, const std::string& name,
     p += "#define PSH_NV " + std::to_string(nv) + "\n";
     p += "#define PSH_OPS " + std::to_string(ops) + "\n";
     p += "#define PSH_ITS " + std::to_string(its) + "\n";
-    p += "#define PSH_STD_TR " + std::to_string(kHookStdTR) + "\n";
-    p += "#define PSH_STD_TC " + std::to_string(kHookStdTC) + "\n";
-    p += "#define PSH_STD_NT " + std::to_string(kHookStdNT) + "\n";
+    p += "#define PSH_BLK_W " + std::to_string(kHookBlkW) + "\n";
+    p += "#define PSH_BLK_NT " + std::to_string(kHookBlkNT) + "\n";
+    p += "#define PSH_BLK_MAXT " + std::to_string(kHookBlkMaxT) + "\n";
     for (const char* ns : kHookNs) {
         p += std::string("namespace ") + ns + " {\n";
         p += "__device__ __constant__ int VARS, TIMES, MPSS, MOSS, NV, OPS, ITS, SX, SY;\n";
@@ -260,9 +292,9 @@ inline int hook_load(HookModule* h, const std::vector<char>& cubin, std::string*
         return -2;
     }
     const char* names[] = {"psh_prism32", "psh_prism64", "psh_gap32", "psh_gap64",
-                           "psh_ybridge", "psh_octahedron", "psh_standard"};
+                           "psh_ybridge", "psh_octahedron", "psh_block"};
     CUfunction* dst[] = {&h->prism[0], &h->prism[1], &h->gap[0], &h->gap[1],
-                         &h->ybridge,  &h->octahedron, &h->standard};
+                         &h->ybridge,  &h->octahedron, &h->block};
     for (int i = 0; i < 7; ++i) {
         r = d.moduleGetFunction(dst[i], h->mod, names[i]);
         if (r == CUDA_SUCCESS)

@@ -12,14 +12,14 @@
 //
 // Here the hook runs inside the same swept phases as the built-in equations
 // (stream_body and seam_body of swept.cuh, with the LINEAR slot layout that
-// keeps the previous, current and next level at one stride) and inside a
-// tiled standard step.  Each kernel kind has its own tile geometry, so the
+// keeps the previous, current and next level at one stride) and inside
+// overlapped blocks.  Each kernel kind has its own tile geometry, so the
 // generated source includes the hook once per kind, in the namespaces
 // psh_stream, psh_seam and psh_std, each with its own framework constants
 // (set by the host before every run) and its own copy of the hook's
 // __constant__ globals (set together by name).  The prelude defines
-// PSH_OPS, PSH_ITS, PSH_NV and the standard tile (PSH_STD_TR x PSH_STD_TC
-// cells, PSH_STD_NT threads) before including this file.
+// PSH_OPS, PSH_ITS, PSH_NV and the block tiles (PSH_BLK_W columns at level 1,
+// PSH_BLK_NT threads, at most PSH_BLK_MAXT levels) before including this file.
 #pragma once
 #include "swept.cuh"
 
@@ -47,13 +47,10 @@ struct HookSeam {
     }
 };
 
-// Standard step tiles: kStdTR x kStdTC cells per CTA, with an OPS-cell
-// periodic halo on every side, three slots (previous, current, next level) of
-// [NV][kStdTR + 2 OPS][kStdTC + 2 OPS] doubles: TIMES = one slot,
-// VARS = one variable plane, SY = one tile row.
-constexpr int kStdTR = PSH_STD_TR, kStdTC = PSH_STD_TC, kStdNT = PSH_STD_NT;
-constexpr int kStdR = kStdTR + 2 * PSH_OPS, kStdC = kStdTC + 2 * PSH_OPS;
-constexpr int kStdSlot = PSH_NV * kStdR * kStdC;
+// Block tiles (psh_block): SX x SY cells per variable with kBlkCols columns,
+// slots of levels -1, 0, 1, .. one after another: TIMES = one slot, VARS = one
+// variable plane, SY = one tile row.
+constexpr int kBlkCols = PSH_BLK_W + 2 * PSH_OPS, kBlkNT = PSH_BLK_NT;
 
 }  // namespace psb
 
@@ -86,41 +83,72 @@ extern "C" __global__ void __launch_bounds__(128) psh_octahedron(SweptArgs a)
     psb::seam_body<psb::HookSeam, PSH_ITS, true, 128, double, true>(a, blockIdx.x, psh_sm);
 }
 
-// One level of the standard decomposition (pysweep/core/pysweep.cu:259-275):
-// the tile of the current and previous level with its periodic halo into
-// shared memory, the hook on every cell, the next level back to the ring
-// (and to a frame when one is due).
-extern "C" __global__ void __launch_bounds__(psb::kStdNT)
-    psh_standard(const double* __restrict__ cur, const double* __restrict__ prev,
-                 double* __restrict__ out, double* __restrict__ frame, int nx, int ny, int gts)
+// T levels of an overlapped block (T = 1: one level of the standard
+// decomposition, pysweep/core/pysweep.cu:259-275).  The tile's newest level (and
+// the one before it, where `older` is given) with a periodic halo of OPS cells
+// per level into shared memory; level m on the rows and columns that are still
+// exact, a warp to a row; the last level's exact cells back (two base levels: the
+// one before it, too), and every level that a frame keeps.  Level 1 spans
+// PSH_BLK_W columns, so that no warp's pass over a row runs nearly empty, and
+// the hook's work is the same on every level: bound by its shared-memory reads
+// (heat: five reads and a write for eight FP64 operations).  Heat as a hook,
+// 200 levels at 1024², prisms of blocksize 16 / here: 3.67 / 0.96 ms.
+struct HookFrames {
+    double* level[PSH_BLK_MAXT];
+};
+
+extern "C" __global__ void __launch_bounds__(psb::kBlkNT)
+    psh_block(const double* __restrict__ newest, const double* __restrict__ older,
+              double* __restrict__ out, double* __restrict__ out1, HookFrames frames, int any_frame,
+              int nx, int ny, int T, int rows1, int gts)
 {
     using namespace psb;
-    constexpr int OPS = PSH_OPS, NV = PSH_NV;
-    extern __shared__ double t[];  // previous, current, next: 3 * kStdSlot
-    const int x0 = blockIdx.y * kStdTR, y0 = blockIdx.x * kStdTC;
+    constexpr int OPS = PSH_OPS, NV = PSH_NV, CC = kBlkCols;
+    constexpr int NP = (CC + 31) / 32;  // passes of a warp over a row
+    extern __shared__ double t[];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, NW = blockDim.x >> 5;
+    const int RR = rows1 + 2 * OPS, SL = NV * RR * CC;  // tile rows, one slot
+    const int ih = rows1 - 2 * OPS * (T - 1), iw = PSH_BLK_W - 2 * OPS * (T - 1);
+    const int x0 = blockIdx.y * ih, y0 = blockIdx.x * iw;
     const size_t vs = (size_t)nx * ny;
-    for (int e = threadIdx.x; e < 2 * kStdSlot; e += kStdNT) {
-        const int s = e / kStdSlot, r = e % kStdSlot;
-        const int v = r / (kStdR * kStdC), i = (r / kStdC) % kStdR, k = r % kStdC;
-        const int x = wrap(x0 + i - OPS, nx), y = wrap(y0 + k - OPS, ny);
-        const double* src = s == 0 ? prev : cur;
-        cp_async8(t + e, src + v * vs + (size_t)x * ny + y);
+    int g[NP];  // grid columns of the lane's tile columns lane + 32 p
+#pragma unroll
+    for (int p = 0; p < NP; ++p) g[p] = wrap(y0 - OPS * T + lane + 32 * p, ny);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int e = w; e < NV * RR; e += NW) {
+        const int v = e / RR, i = e % RR;
+        const size_t o = v * vs + (size_t)wrap(x0 - OPS * T + i, nx) * ny;
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            const int k = lane + 32 * p;
+            if (k < CC) {
+                cp_async8(t + SL + e * CC + k, newest + o + g[p]);
+                if (older) cp_async8(t + e * CC + k, older + o + g[p]);
+            }
+        }
     }
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
-    for (int c = threadIdx.x; c < kStdTR * kStdTC; c += kStdNT) {
-        const int i = c / kStdTC, k = c % kStdTC;
-        if (x0 + i < nx && y0 + k < ny)
-            psh_std::step(t, kStdSlot + (i + OPS) * kStdC + k + OPS, gts);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // the exact cells of level m to global memory
+    auto store = [&](double* dst, int m) {
+        const double* src = t + (m + 1) * SL;
+        for (int e = w; e < NV * ih; e += NW) {
+            const int v = e / ih, i = e % ih;
+            if (x0 + i >= nx) continue;
+            double* row = dst + v * vs + (size_t)(x0 + i) * ny + y0;
+            const double* from = src + (v * RR + i + OPS * T) * CC + OPS * T;
+            for (int k = lane; k < iw && y0 + k < ny; k += 32) row[k] = from[k];
+        }
+    };
+    for (int m = 1; m <= T; ++m) {
+        const int lo = OPS * m;
+        for (int i = lo + w; i < RR - lo; i += NW)
+            for (int k = lo + lane; k < CC - lo; k += 32) psh_std::step(t, m * SL + i * CC + k, gts + m - 1);
+        __syncthreads();
+        if (any_frame && frames.level[m - 1]) store(frames.level[m - 1], m);
     }
-    __syncthreads();
-    for (int c = threadIdx.x; c < NV * kStdTR * kStdTC; c += kStdNT) {
-        const int v = c / (kStdTR * kStdTC), i = (c / kStdTC) % kStdTR, k = c % kStdTC;
-        if (x0 + i >= nx || y0 + k >= ny) continue;
-        const double val = t[2 * kStdSlot + (v * kStdR + i + OPS) * kStdC + k + OPS];
-        const size_t go = v * vs + (size_t)(x0 + i) * ny + y0 + k;
-        out[go] = val;
-        if (frame) frame[go] = val;
-    }
+    store(out, T);
+    if (out1) store(out1, T - 1);
 }

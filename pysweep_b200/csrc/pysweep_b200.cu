@@ -811,6 +811,78 @@ int run_march(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
                       });
 }
 
+struct HookFrames {  // psh_block's argument (hook_kernels.cuh)
+    double* level[kHookBlkMaxT];
+};
+
+// Queue one psh_block launch of T levels (its launch may overlap the end of the
+// one before it).
+void hook_block_launch(ps_solver* s, const HookBlock& b, int T, const double* newest,
+                       const double* older, double* out, double* out1, HookFrames fr, int any_frame,
+                       int gts)
+{
+    int nx = s->nx, ny = s->ny, rows = b.rows;
+    const int ih = rows - 2 * s->ops * (T - 1), iw = kHookBlkW - 2 * s->ops * (T - 1);
+    void* args[] = {&newest, &older, &out, &out1, &fr, &any_frame, &nx, &ny, &T, &rows, &gts};
+    CUlaunchConfig cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDimX = (ny + iw - 1) / iw;
+    cfg.gridDimY = (nx + ih - 1) / ih;
+    cfg.gridDimZ = 1;
+    cfg.blockDimX = hook_block_threads(T);
+    cfg.blockDimY = cfg.blockDimZ = 1;
+    cfg.sharedMemBytes = (unsigned)hook_block_smem(s->nv, s->ops, rows, T);
+    cfg.hStream = (CUstream)s->stream;
+    CUlaunchAttribute at;
+    memset(&at, 0, sizeof at);
+    at.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+    at.value.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    CUresult r = drv().launchKernelEx(&cfg, s->hook->block, args, nullptr);
+    if (r != CUDA_SUCCESS) s->launch_err = cu_error(r);
+}
+
+// The framework constants of the block tiles (the same for any T).
+int hook_block_frame(ps_solver* s, const HookBlock& b)
+{
+    const int rr = b.rows + 2 * s->ops, cc = kHookBlkW + 2 * s->ops;
+    return hook_frame(s, HOOK_STD, rr, cc, s->nv * rr * cc);
+}
+
+// A step hook in overlapped blocks.
+int run_hook_block(ps_solver* s, const HookBlock& b, int64_t nlevels, int gts0, double* frames,
+                   int64_t frame_cap, int frame_every)
+{
+    const size_t fe = field_elems(s);
+    const int its = s->its, every = frame_every > 0 ? frame_every : 1;
+    int rc = hook_block_frame(s, b);
+    if (rc) return rc;
+    for (int64_t done = 0; done < nlevels;) {
+        const int64_t left = nlevels - done, k = (left + b.T - 1) / b.T;
+        const int T = (int)((left + k - 1) / k);  // even shares
+        HookFrames fr = {};
+        int any = 0;
+        for (int m = 1; m <= T; ++m) {
+            const int64_t L = done + m;
+            if (!frames || L % its || (L / its) % every || (L / its) / every - 1 >= frame_cap) continue;
+            fr.level[m - 1] = at(s, frames, (size_t)((L / its) / every - 1) * fe);
+            any = 1;
+        }
+        double* in = s->base[s->cur];
+        double* out = s->base[1 - s->cur];
+        if ((rc = timed_launch(s, 5, (double)s->nx * s->ny * T, [&] {
+                 hook_block_launch(s, b, T, at(s, in, (size_t)(its - 1) * fe), its == 2 ? in : nullptr,
+                                   at(s, out, (size_t)(its - 1) * fe), its == 2 ? out : nullptr, fr,
+                                   any, gts0 + (int)done);
+             })))
+            return rc;
+        s->cur = 1 - s->cur;
+        done += T;
+    }
+    return PS_OK;
+}
+
 template <bool RK2, class T>
 int run_heat_standard(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t frame_cap,
                       int frame_every)
@@ -944,6 +1016,10 @@ int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
         // (frames that 4-wide stores cannot reach may fall on half stages)
         if (maxT >= 2 && aligned32(frames))
             return run_block<double, true>(s, nlevels, gts0, frames, frame_cap, frame_every, maxT);
+    }
+    if (s->hook && s->threads != 256) {
+        const HookBlock b = hook_block(s->nv, s->ops, s->h_set ? s->H : kHookBlkMaxT);
+        if (b.rows) return run_hook_block(s, b, nlevels, gts0, frames, frame_cap, frame_every);
     }
     if (s->eq == PS_EQ_EULER && s->threads != 256 && march_constants(make_params(s)))
         return run_march(s, nlevels, gts0, frames, frame_cap, frame_every, 5);
@@ -1090,11 +1166,11 @@ int run_standard(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_
     const EqParams prm = make_params(s);
     const int every = frame_every > 0 ? frame_every : 1;
     int rc;
+    HookBlock blk{};
     if (s->hook) {
-        // the hook's standard tile: kHookStdTR x kHookStdTC cells and an
-        // OPS-cell halo per variable, previous / current / next level one slot apart
-        const int tr = kHookStdTR + 2 * s->ops, tc = kHookStdTC + 2 * s->ops;
-        if ((rc = hook_frame(s, HOOK_STD, tr, tc, s->nv * tr * tc))) return rc;
+        blk = hook_block(s->nv, s->ops, 1);
+        if (!blk.rows) return fail(s, PS_ERR_UNSUPPORTED, "the hook's standard tile does not fit in shared memory");
+        if ((rc = hook_block_frame(s, blk))) return rc;
     }
     for (int64_t L = 1; L <= nlevels; ++L) {
         double* fr = nullptr;
@@ -1105,15 +1181,9 @@ int run_standard(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_
         const int gts = gts0 + (int)(L - 1);
         if ((rc = timed_launch(s, 4, (double)s->nx * s->ny, [&] {
                  if (s->hook) {
-                     const double* cur = s->ring[c];
-                     const double* prv = s->ring[p];
-                     double* nxt = s->ring[n];
-                     int nx = s->nx, ny = s->ny, g = gts;
-                     void* args[] = {&cur, &prv, &nxt, &fr, &nx, &ny, &g};
-                     const size_t tr = kHookStdTR + 2 * s->ops, tc = kHookStdTC + 2 * s->ops;
-                     hook_launch(s, s->hook->standard, (s->ny + kHookStdTC - 1) / kHookStdTC,
-                                 (s->nx + kHookStdTR - 1) / kHookStdTR, kHookStdNT,
-                                 3 * sizeof(double) * s->nv * tr * tc, s->stream, args);
+                     HookFrames f = {};
+                     f.level[0] = fr;
+                     hook_block_launch(s, blk, 1, s->ring[c], s->ring[p], s->ring[n], nullptr, f, fr != nullptr, gts);
                  } else {
                      K(s->ring[c], s->ring[p], s->ring[n], fr, s->nx, s->ny, s->nv, gts, prm,
                        s->stream);
