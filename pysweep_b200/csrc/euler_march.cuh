@@ -158,7 +158,7 @@ __device__ __noinline__ void face_plain(double gamma, double gm1, const double* 
 }
 
 // Two faces, each between cells a and b (q and the factor of the side towards
-// the face): flux f and spectral term s, the values of face() in
+// the face): flux f and spectral term s, the values of flux and spectral in
 // equations.cuh.  plain: some state of the warp's is out of the safe range.
 template <int DIR>
 __device__ __forceinline__ void faces2(bool plain, double gamma, double gm1,
@@ -422,6 +422,40 @@ __global__ void __launch_bounds__(32, kMarchWarps) euler_march(const __grid_cons
 {
     __shared__ __align__(16) MarchShared sh;
     march_body(a, blockIdx.x, sh);
+}
+
+// Many instances in one launch: block g is unit units[g].y of instance
+// units[g].x.  slot: the level's place in an instance's base buffers, [base][2]
+// fields; an instance counts its own levels.
+struct MarchInst {
+    double* base[2];
+    double dtdx, dtdy, gamma, gm1;
+    int nx, ny, level;
+};
+
+__global__ void __launch_bounds__(32, kMarchWarps)
+    euler_march_batch(const MarchInst* __restrict__ inst, const int2* __restrict__ units, int cur,
+                      int prev, int out, int hs, int L)
+{
+    __shared__ __align__(16) MarchShared sh;
+    const int2 u = units[blockIdx.x];
+    const MarchInst b = inst[u.x];
+    const size_t fe = (size_t)4 * b.nx * b.ny;
+    MarchArgs a;
+    a.cur = b.base[cur / 2] + cur % 2 * fe;
+    a.prev = b.base[prev / 2] + prev % 2 * fe;
+    a.out = b.base[out / 2] + out % 2 * fe;
+    a.frame = nullptr;
+    a.nx = b.nx;
+    a.ny = b.ny;
+    a.ncs = (b.ny + kMarchW - 1) / kMarchW;
+    a.hs = hs;
+    a.gts = b.level + L;
+    a.dtdx = b.dtdx;
+    a.dtdy = b.dtdy;
+    a.gamma = b.gamma;
+    a.gm1 = b.gm1;
+    march_body(a, u.y, sh);
 }
 
 // Rows of a strip: one wave of warps.

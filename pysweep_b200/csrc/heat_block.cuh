@@ -35,7 +35,8 @@
 #include <algorithm>
 #include <type_traits>
 
-#include "heat_fast.cuh"
+#include "heat_cell.cuh"
+#include "launch.cuh"
 
 namespace psb {
 
@@ -571,6 +572,46 @@ inline int plan_next(const BlockPlan& p, long long left, int step)
     if (p.stream) return left >= kStreamT ? kStreamT : (int)((left + step - 1) / step * step);
     const long long k = (left + p.T - 1) / p.T;
     return (int)(((left + k - 1) / k + step - 1) / step * step);
+}
+
+// --------------------------------------------------------------- launches --
+template <class S, bool RK2, int C, int R, int MAXW>
+inline void launch_tile(const BlockArgs& a, int nw, cudaStream_t st)
+{
+    auto k = heat_block_tile<S, RK2, C, R, MAXW>;
+    const size_t smem = tile_smem<C>(nw);
+    if (smem > 48 * 1024) allow_big_smem(k);
+    launch_after(k, a.units, 32 * nw, smem, st, a);
+}
+
+template <class S, bool RK2>
+inline void launch_block_tile(const TileShape& t, BlockArgs a, int T, cudaStream_t st)
+{
+    a.T = T;
+    a.vw = tile_vw(t, T);
+    a.vh = tile_vh(t, T);
+    a.ncs = (a.ny + a.vw - 1) / a.vw;
+    a.units = a.ncs * ((a.nx + a.vh - 1) / a.vh);
+    if constexpr (RK2) {
+        if (t.C == 4) launch_tile<S, RK2, 4, 4, 16>(a, t.nw, st);
+        else launch_tile<S, RK2, 2, 4, 24>(a, t.nw, st);
+    } else {
+        if (t.C == 4) launch_tile<S, RK2, 4, 6, 16>(a, t.nw, st);
+        else if (t.R == 8) launch_tile<S, RK2, 2, 8, 20>(a, t.nw, st);
+        else launch_tile<S, RK2, 2, 4, 24>(a, t.nw, st);
+    }
+}
+
+template <class S, bool RK2>
+inline void launch_block_stream(BlockArgs a, int sms, cudaStream_t st)
+{
+    a.T = kStreamT;
+    a.vw = kStreamW;
+    a.ncs = (a.ny + a.vw - 1) / a.vw;
+    const BlockGrid g{a.nx, a.ny};
+    a.vh = stream_rows(BlockGrids{&g, 1}, sms);
+    a.units = a.ncs * ((a.nx + a.vh - 1) / a.vh);
+    launch_after(heat_block_stream<S, RK2>, a.units, 32, 0, st, a);
 }
 
 // ------------------------------------------------------------------ batch --

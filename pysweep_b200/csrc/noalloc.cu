@@ -15,9 +15,7 @@
 #include <mutex>
 
 #include "../../include/pysweep_b200.h"
-#include "heat_fast.cuh"
-#include "seam_fast.cuh"
-#include "swept.cuh"
+#include "heat_block.cuh"
 
 namespace {
 
@@ -61,25 +59,24 @@ extern "C" int ps_heat_swept_noalloc(const double* d_in, double* d_out, int nx, 
         return PS_ERR_INVALID;
     }
     if ((blocksize != 16 && blocksize != 32) || nx <= 0 || ny <= 0 || nx % blocksize ||
-        ny % kFastChunk || nsteps < 0) {
+        ny % 64 || nsteps < 0) {
         snprintf(msg, sizeof msg,
                  "need blocksize 16 or 32, nx a multiple of it, ny a multiple of %d, nsteps >= 0 "
                  "(got bs %d, %dx%d, %lld steps)",
-                 kFastChunk, blocksize, nx, ny, (long long)nsteps);
+                 64, blocksize, nx, ny, (long long)nsteps);
         put_err(err, errlen, msg);
         return PS_ERR_INVALID;
     }
     cudaStream_t st = (cudaStream_t)stream;
     const size_t fe = (size_t)nx * ny;
-    // tiling: the defaults of a ps_solver (MPSS levels per half-cycle, one
-    // wave of warps); results do not depend on it
     int dev = 0;
     cudaGetDevice(&dev);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int BX = blocksize, H = BX / 2 - 1, HF = H - 1, nb = nx / BX;
-    const int nseg =
-        std::max(1, std::min(ny / kFastChunk, sms * fast_ctas_per_sm(BX, 0) * kFastWarps / nb));
+    // the sizes this entry point has always taken: a field and the faces of a
+    // prism decomposition in the scratch array (blocks need the field only)
+    const int BX = blocksize, HF = BX / 2 - 2, nb = nx / BX;
+    const int nseg = std::max(1, std::min(ny / 64, sms * (BX == 16 ? 16 : 12) / nb));
     const size_t field_b = round_up(fe * sizeof(double));
     const size_t xface_b = round_up((size_t)nb * HF * 2 * 2 * ny * sizeof(double));
     const size_t yface_b = round_up((size_t)nb * nseg * 2 * HF * BX * 2 * sizeof(double));
@@ -122,19 +119,6 @@ extern "C" int ps_heat_swept_noalloc(const double* d_in, double* d_out, int nx, 
                 put_err(err, errlen, msg);
                 return PS_ERR_CUDA;
             }
-            const void* kernels[] = {
-                (const void*)heat_stream_fast<16, false>, (const void*)heat_stream_fast<16, true>,
-                (const void*)heat_stream_fast<32, false>, (const void*)heat_stream_fast<32, true>,
-                (const void*)heat_yseam_fast<16>, (const void*)heat_oseam_fast<16>,
-                (const void*)heat_yseam_fast<32>, (const void*)heat_oseam_fast<32>};
-            for (const void* k : kernels) {
-                e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-                if (e != cudaSuccess) {
-                    snprintf(msg, sizeof msg, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-                    put_err(err, errlen, msg);
-                    return PS_ERR_CUDA;  // the device stays unset: the next call retries
-                }
-            }
             g_scratch_ptr[dev] = p;
         }
         base = g_scratch_ptr[dev];
@@ -144,68 +128,37 @@ extern "C" int ps_heat_swept_noalloc(const double* d_in, double* d_out, int nx, 
         put_err(err, errlen, "d_in or d_out lies inside the library's scratch array");
         return PS_ERR_INVALID;
     }
-    double* A = (double*)base;
-    SweptArgs a;
+    // Overlapped blocks (heat_block.cuh), the launches and kernels of ps_run.
+    // Outputs alternate between d_out and the scratch field so that the last
+    // launch lands in d_out and d_in is only read
+    const BlockGrid grid{nx, ny};
+    const BlockGrids grids{&grid, 1};
+    const BlockPlan plan = plan_block(kTilesFE, grids, (int)std::min<int64_t>(nsteps, 1 << 20), 1,
+                                      kTileMaxT, sms);
+    int64_t count = 0;
+    for (int64_t done = 0; done < nsteps; ++count) done += plan_next(plan, nsteps - done, 1);
+    BlockArgs a;
     memset(&a, 0, sizeof a);
     a.nx = nx;
     a.ny = ny;
-    a.nv = 1;
-    a.bx = BX;
-    a.hx = BX / 2;
-    a.Hmax = H;
-    a.nb = nb;
-    a.nseg = nseg;
-    a.wy = ny / nseg;
-    a.nchunks = a.wy / kFastChunk;
-    a.seg_unit = 32;
-    a.seg_units = ny / 32;
-    a.its = 1;
-    a.gts_base = 0;
-    a.frame_every = 1;
-    a.xface = (double*)((unsigned char*)base + field_b);
-    a.yface = (double*)((unsigned char*)base + field_b + xface_b);
-    a.p.d[0] = alpha * dt / dx / dx;  // heat.py:37
-    a.p.i[0] = 1;                     // forward Euler
-    const int units = nb * nseg;
-    const int fgrid = (units + kFastWarps - 1) / kFastWarps;
-    const size_t fsm = BX == 16 ? heat_fast_smem<16>(H) : heat_fast_smem<32>(H);
-    // the register seams: one warp per block edge
-    const int sgrid = (units + kSeamWarps - 1) / kSeamWarps;
-    const size_t ssm = BX == 16 ? yseam_smem<16>(H) : yseam_smem<32>(H);
-    const int64_t halves = (nsteps + H - 1) / H;
-    // outputs alternate between d_out and the scratch field so that the last
-    // half-cycle lands in d_out and d_in is only read
-    const double* in = d_in;
+    a.v4 = (uintptr_t)d_in % 32 == 0 && (uintptr_t)d_out % 32 == 0;
+    a.cr = alpha * dt / dx / dx;  // heat.py:37
+    a.in = d_in;
     int64_t done = 0;
-    int off = 0;
-    for (int64_t t = 0; t < halves; ++t) {
-        const int h = (int)std::min<int64_t>(H, nsteps - done);
-        double* out = ((halves - 1 - t) % 2 == 0) ? d_out : A;
-        a.H = h;
-        a.L0 = done;
-        a.off = off;
-        a.bin = in;
-        a.bout = out;
-        if (BX == 16) {
-            heat_stream_fast<16, false><<<fgrid, 32 * kFastWarps, fsm, st>>>(a);
-            heat_yseam_fast<16><<<sgrid, 32 * kSeamWarps, ssm, st>>>(a);
-            heat_stream_fast<16, true><<<fgrid, 32 * kFastWarps, fsm, st>>>(a);
-            heat_oseam_fast<16><<<sgrid, 32 * kSeamWarps, ssm, st>>>(a);
-        } else {
-            heat_stream_fast<32, false><<<fgrid, 32 * kFastWarps, fsm, st>>>(a);
-            heat_yseam_fast<32><<<sgrid, 32 * kSeamWarps, ssm, st>>>(a);
-            heat_stream_fast<32, true><<<fgrid, 32 * kFastWarps, fsm, st>>>(a);
-            heat_oseam_fast<32><<<sgrid, 32 * kSeamWarps, ssm, st>>>(a);
-        }
+    for (int64_t k = 0; k < count; ++k) {
+        const int T = plan_next(plan, nsteps - done, 1);
+        a.out = (count - 1 - k) % 2 == 0 ? d_out : (double*)base;
+        double us;
+        if (plan.stream && T == kStreamT) launch_block_stream<double, false>(a, sms, st);
+        else launch_block_tile<double, false>(best_tile(kTilesFE, T, grids, sms, &us), a, T, st);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
             snprintf(msg, sizeof msg, "kernel launch: %s", cudaGetErrorString(e));
             put_err(err, errlen, msg);
             return PS_ERR_CUDA;
         }
-        in = out;
-        off = ((off - BX / 2) % nx + nx) % nx;
-        done += h;
+        a.in = a.out;
+        done += T;
     }
     return PS_OK;
 }

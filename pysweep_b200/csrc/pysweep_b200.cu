@@ -14,8 +14,6 @@
 #include "../../include/pysweep_b200.h"
 #include "equations.cuh"
 #include "swept.cuh"
-#include "heat_fast.cuh"
-#include "seam_fast.cuh"
 #include "heat_block.cuh"
 #include "heatvar_block.cuh"
 #include "launch.cuh"
@@ -228,14 +226,14 @@ void launch_stream(const SweptArgs& a, int grid, size_t smem, cudaStream_t st)
     k<<<grid, 256, smem, st>>>(a);
 }
 
-template <class Eq, int ITS, bool GAP, class T = double>
+template <class Eq, int ITS, bool GAP>
 void launch_seam(const SweptArgs& a, int grid, size_t smem, cudaStream_t st)
 {
     // one-variable stencils: 64 threads per seam (the seams are issue-bound
     // on per-level loop work that every warp repeats; measured 1-2% faster
     // in total than 128); Euler keeps 128 for its four-variable tiles
     constexpr int NT = Eq::OPS == 1 ? 64 : 128;
-    auto k = seam_kernel<Eq, ITS, GAP, NT, T>;
+    auto k = seam_kernel<Eq, ITS, GAP, NT>;
     allow_big_smem(k);
     k<<<grid, NT, smem, st>>>(a);
 }
@@ -250,40 +248,7 @@ void launch_standard(const double* cur, const double* prev, double* out, double*
 
 struct SweptSet {
     SweptLaunch P, Y, G, O;
-    bool fast = false;
 };
-
-template <int BX, bool GAP, class T = double, int VAR = 0, int MINROWS = 2>
-void launch_fast(const SweptArgs& a, int grid, size_t smem, cudaStream_t st)
-{
-    auto k = heat_stream_fast<BX, GAP, T, VAR, MINROWS>;
-    allow_big_smem(k);
-    const int units = a.nb * a.nseg;
-    // the per-cell courant variants add their operand ring to each warp's share
-    if (VAR) smem = heat_fast_smem_v<BX, VAR>(a.Hmax);
-    k<<<(units + kFastWarps - 1) / kFastWarps, 32 * kFastWarps, smem, st>>>(a);
-}
-
-// register-resident y-bridge seams of heat (seam_fast.cuh): one warp per
-// column edge, the staged y-faces in shared memory
-template <int BX>
-void launch_yseam(const SweptArgs& a, int grid, size_t, cudaStream_t st)
-{
-    auto k = heat_yseam_fast<BX>;
-    allow_big_smem(k);
-    const int units = a.nb * a.nseg;
-    k<<<(units + kSeamWarps - 1) / kSeamWarps, 32 * kSeamWarps, yseam_smem<BX>(a.Hmax), st>>>(a);
-}
-
-// register-resident octahedron seams of heat (seam_fast.cuh)
-template <int BX>
-void launch_oseam(const SweptArgs& a, int grid, size_t, cudaStream_t st)
-{
-    auto k = heat_oseam_fast<BX>;
-    allow_big_smem(k);
-    const int units = a.nb * a.nseg;
-    k<<<(units + kSeamWarps - 1) / kSeamWarps, 32 * kSeamWarps, yseam_smem<BX>(a.Hmax), st>>>(a);
-}
 
 template <class Eq, int ITS, int W>
 SweptSet make_set()
@@ -293,10 +258,6 @@ SweptSet make_set()
 }
 
 // (equation, ops, its, chunk) -> kernels; nullptr members = not built.
-// Euler's stream tiles with the per-cell step (see EulerCell): an internal
-// equation id for kernel selection only
-constexpr int PS_EQ_EULER_CELL = 100;
-
 bool pick_swept(int eq, int ops, int its, int chunk, SweptSet* out)
 {
 #define PS_SET(EQ, OP, IT, W, T) \
@@ -307,8 +268,6 @@ bool pick_swept(int eq, int ops, int its, int chunk, SweptSet* out)
     PS_SET(PS_EQ_HEAT, 1, 2, 64, Heat)
     PS_SET(PS_EQ_EULER, 2, 2, 32, Euler)
     PS_SET(PS_EQ_EULER, 2, 2, 64, Euler)
-    PS_SET(PS_EQ_EULER_CELL, 2, 2, 32, EulerCell)
-    PS_SET(PS_EQ_EULER_CELL, 2, 2, 64, EulerCell)
     PS_SET(PS_EQ_HALF, 1, 1, 32, Half)
     PS_SET(PS_EQ_HALF, 1, 2, 32, Half)
     PS_SET(PS_EQ_EXAMPLE, 1, 1, 32, ExampleT<1>)
@@ -450,29 +409,13 @@ int default_levels(int eq, int its, int bs, int mpss)
 // equations, levels -1 .. Hmax for a step hook (slot_count in swept.cuh)
 int tile_slots(const ps_solver* s) { return s->hook ? s->H + 2 : s->its + 1; }
 
-size_t stream_tile_smem(const ps_solver* s)
+size_t stream_smem(const ps_solver* s)
 {
     const int O2 = 2 * s->ops, RS = s->chunk + O2;
     return s->esize * ((size_t)tile_slots(s) * s->nv * s->bs * RS +
                        (size_t)(s->H + 1) * s->nv * s->bs * O2);
 }
 
-// Euler streams share faces between cells when tile and scratch still leave
-// room for two CTAs per SM (measured: with one CTA per SM the per-cell step
-// on a wider chunk is faster; Euler stream levels are latency-bound)
-constexpr size_t kFaceSmemCap = 113 * 1024;
-bool euler_faces_fit(const ps_solver* s)
-{
-    return s->eq == PS_EQ_EULER &&
-           stream_tile_smem(s) + sizeof(double) * euler_level_scratch(s->bs, s->chunk) <=
-               kFaceSmemCap;
-}
-
-size_t stream_smem(const ps_solver* s)
-{
-    return stream_tile_smem(s) +
-           (euler_faces_fit(s) ? sizeof(double) * euler_level_scratch(s->bs, s->chunk) : 0);
-}
 
 bool solver_seam_direct(const ps_solver* s)
 {
@@ -530,45 +473,6 @@ int hook_frame(ps_solver* s, int ns, int rows, int cols, int times)
 }
 
 // ------------------------------------------------- overlapped heat blocks ----
-template <class S, bool RK2, int C, int R, int MAXW>
-void launch_tile(const BlockArgs& a, int nw, cudaStream_t st)
-{
-    auto k = heat_block_tile<S, RK2, C, R, MAXW>;
-    const size_t smem = tile_smem<C>(nw);
-    if (smem > 48 * 1024) allow_big_smem(k);
-    launch_after(k, a.units, 32 * nw, smem, st, a);
-}
-
-template <class S, bool RK2>
-void launch_block_tile(const TileShape& t, BlockArgs a, int T, cudaStream_t st)
-{
-    a.T = T;
-    a.vw = tile_vw(t, T);
-    a.vh = tile_vh(t, T);
-    a.ncs = (a.ny + a.vw - 1) / a.vw;
-    a.units = a.ncs * ((a.nx + a.vh - 1) / a.vh);
-    if constexpr (RK2) {
-        if (t.C == 4) launch_tile<S, RK2, 4, 4, 16>(a, t.nw, st);
-        else launch_tile<S, RK2, 2, 4, 24>(a, t.nw, st);
-    } else {
-        if (t.C == 4) launch_tile<S, RK2, 4, 6, 16>(a, t.nw, st);
-        else if (t.R == 8) launch_tile<S, RK2, 2, 8, 20>(a, t.nw, st);
-        else launch_tile<S, RK2, 2, 4, 24>(a, t.nw, st);
-    }
-}
-
-template <class S, bool RK2>
-void launch_block_stream(BlockArgs a, int sms, cudaStream_t st)
-{
-    a.T = kStreamT;
-    a.vw = kStreamW;
-    a.ncs = (a.ny + a.vw - 1) / a.vw;
-    const BlockGrid g{a.nx, a.ny};
-    a.vh = stream_rows(BlockGrids{&g, 1}, sms);
-    a.units = a.ncs * ((a.nx + a.vh - 1) / a.vh);
-    launch_after(heat_block_stream<S, RK2>, a.units, 32, 0, st, a);
-}
-
 bool aligned32(const void* p) { return reinterpret_cast<uintptr_t>(p) % 32 == 0; }
 
 // Heat through overlapped space-time blocks (heat_block.cuh): forward Euler
@@ -905,81 +809,46 @@ int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
               int frame_every)
 {
     SweptSet K;
-    const int keq = (s->eq == PS_EQ_EULER && !euler_faces_fit(s)) ? PS_EQ_EULER_CELL : s->eq;
     if (s->hook) {
         K = hook_set(s);
-    } else if (!pick_swept(keq, s->ops, s->its, s->chunk, &K)) {
+    } else if (!pick_swept(s->eq, s->ops, s->its, s->chunk, &K)) {
         return fail(s, PS_ERR_UNSUPPORTED, "no swept kernels for equation %d ops %d its %d chunk %d",
                     s->eq, s->ops, s->its, s->chunk);
     }
     const int O2 = 2 * s->ops;
-    // register-resident streams for heat with forward Euler (the generic
-    // seam kernels are shared)
     const bool fwd_euler = make_params(s).i[0] != 0;
-    if (s->dtype == PS_DTYPE_F32) {
-        // float32 fields: the register streams and the seams in float storage
-        if (!(s->eq == PS_EQ_HEAT && s->its == 1 && fwd_euler && (s->bs == 16 || s->bs == 32) &&
-              s->ny % 32 == 0))
-            return fail(s, PS_ERR_UNSUPPORTED,
-                        "float32 fields: heat, forward Euler, blocksize 16 or 32, ny a multiple of 32");
-        K.fast = true;
-        K.Y = launch_seam<HeatF32, 1, false, float>;
-        K.O = launch_seam<HeatF32, 1, true, float>;
-        K.P = s->bs == 16 ? launch_fast<16, false, float> : launch_fast<32, false, float>;
-        K.G = s->bs == 16 ? launch_fast<16, true, float> : launch_fast<32, true, float>;
-    } else if (!s->hook && s->eq == PS_EQ_HEAT && s->its == 1 && fwd_euler && s->threads != 256 &&
-               (s->bs == 16 || s->bs == 32) && s->ny % 32 == 0) {
-        K.fast = true;
-        if (s->bs == 16) {
-            K.P = launch_fast<16, false>;
-            K.G = launch_fast<16, true>;
-            K.Y = launch_yseam<16>;
-            K.O = launch_oseam<16>;
-        } else {
-            // at most 14 levels per half-cycle: every prism level keeps 4 rows
-            // or more, so its first 4 rows need no end test (8192², 1200
-            // levels: 0.577 -> 0.570 ms per launch; 8 rows spilled)
-            K.P = s->H <= 14 ? launch_fast<32, false, double, 0, 4> : launch_fast<32, false>;
-            K.G = launch_fast<32, true>;
-            K.Y = launch_yseam<32>;
-            K.O = launch_oseam<32>;
-        }
-    } else if ((s->eq == PS_EQ_HEATVAR || s->eq == PS_EQ_HEATVAR_ADJMU) && s->threads != 256 &&
-               (s->bs == 16 || s->bs == 32) && s->ny % 32 == 0) {
-        // per-cell courant numbers in the register streams (the seams: the
-        // generic kernels with the same equation's step_at)
-        K.fast = true;
-        if (s->eq == PS_EQ_HEATVAR) {
-            K.P = s->bs == 16 ? launch_fast<16, false, double, 1> : launch_fast<32, false, double, 1>;
-            K.G = s->bs == 16 ? launch_fast<16, true, double, 1> : launch_fast<32, true, double, 1>;
-        } else {
-            K.P = s->bs == 16 ? launch_fast<16, false, double, 2> : launch_fast<32, false, double, 2>;
-            K.G = s->bs == 16 ? launch_fast<16, true, double, 2> : launch_fast<32, true, double, 2>;
-        }
-    }
+    const bool var = s->eq == PS_EQ_HEATVAR || s->eq == PS_EQ_HEATVAR_ADJMU;
+    const bool shape = (s->bs == 16 || s->bs == 32) && s->ny % 32 == 0;
+    if (s->dtype == PS_DTYPE_F32 && !(s->eq == PS_EQ_HEAT && s->its == 1 && fwd_euler && shape))
+        return fail(s, PS_ERR_UNSUPPORTED,
+                    "float32 fields: heat, forward Euler, blocksize 16 or 32, ny a multiple of 32");
+    // Column segments of any count up to ny/32 for heat and its
+    // variable-courant form on these shapes (they run in blocks of their own
+    // size: the count is only reported); divisors of ny for the prisms
+    const bool free_seg = s->dtype == PS_DTYPE_F32 ||
+                          (shape && s->threads != 256 &&
+                           ((s->eq == PS_EQ_HEAT && s->its == 1 && fwd_euler) || var));
     if (s->H < 1 || s->H > s->mpss) return fail(s, PS_ERR_INVALID, "levels per half-cycle %d not in [1, %d]", s->H, s->mpss);
     if (s->chunk < O2 * (s->H + 1))
         return fail(s, PS_ERR_INVALID, "chunk %d narrower than 2*ops*(h+1) = %d", s->chunk, O2 * (s->H + 1));
-    if (K.fast) {
+    if (free_seg) {
         if (s->nseg < 1 || s->nseg > s->ny / 32)
             return fail(s, PS_ERR_INVALID, "nseg %d not in [1, ny/32 = %d]", s->nseg, s->ny / 32);
     } else if (s->nseg < 1 || s->ny % s->nseg) {
         return fail(s, PS_ERR_INVALID, "ny %d not divisible into %d segments", s->ny, s->nseg);
     }
     // the first chunk of a segment shrinks by 2*ops per level on its left edge
-    if (!K.fast && std::min(s->chunk, s->ny / s->nseg) < O2 * (s->H + 1))
+    if (!free_seg && std::min(s->chunk, s->ny / s->nseg) < O2 * (s->H + 1))
         return fail(s, PS_ERR_INVALID, "segment width %d narrower than 2*ops*(h+1) = %d",
                     s->ny / s->nseg, O2 * (s->H + 1));
     if (s->nseg_auto) {
-        if (K.fast) {
-            // one warp per (band, segment); as many as the CTAs of 4 warps
-            // that fit on the SMs at once (fast_ctas_per_sm)
+        if (free_seg) {
+            // as many as 12 warps per SM have bands (8 with a courant number
+            // per cell, 16 of 16 rows), of 64 columns or more
             int sms = 148;
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-            const bool var = s->eq == PS_EQ_HEATVAR || s->eq == PS_EQ_HEATVAR_ADJMU;
-            const int slots = sms * fast_ctas_per_sm(s->bs, var ? 1 : 0) * kFastWarps;
-            const int nb = s->nx / s->bs;
-            s->nseg = std::max(1, std::min(s->ny / kFastChunk, slots / nb));
+            const int warps = s->bs == 16 ? 16 : (var ? 8 : 12);
+            s->nseg = std::max(1, std::min(s->ny / 64, sms * warps / (s->nx / s->bs)));
             s->nseg = std::max(1, std::min(s->nseg, s->ny / 32));
         } else {
             // one CTA per (band, segment): the most segments that divide ny
@@ -1005,9 +874,10 @@ int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
     const size_t smem = std::max(stream_smem(s), seam_smem(s));
     if (smem > 227 * 1024)
         return fail(s, PS_ERR_UNSUPPORTED, "tile needs %zu bytes of shared memory", smem);
-    // heat in overlapped blocks; threads 256 keeps the shared-memory prisms,
-    // and a configured h bounds the levels of a launch
-    if (!s->hook && s->eq == PS_EQ_HEAT && s->threads != 256 && (s->its == 1) == fwd_euler) {
+    // heat in overlapped blocks; threads 256 keeps the shared-memory prisms
+    // (float64), and a configured h bounds the levels of a launch
+    if (!s->hook && s->eq == PS_EQ_HEAT && (s->threads != 256 || s->dtype == PS_DTYPE_F32) &&
+        (s->its == 1) == fwd_euler) {
         const int maxT = s->h_set ? s->H : kTileMaxT;
         if (s->dtype == PS_DTYPE_F32)
             return run_block<float, false>(s, nlevels, gts0, frames, frame_cap, frame_every, maxT);
@@ -1054,13 +924,12 @@ int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
     a.hx = s->bs / 2;
     a.Hmax = s->H;
     a.nb = s->nx / s->bs;
-    a.nseg = s->nseg;
-    a.wy = s->ny / s->nseg;
-    // the last chunk may be partial (generic streams); the register streams
-    // use whole 64-column chunks
-    a.nchunks = K.fast ? a.wy / kFastChunk : (a.wy + s->chunk - 1) / s->chunk;
-    a.seg_unit = K.fast ? 32 : a.wy;
-    a.seg_units = K.fast ? s->ny / 32 : s->nseg;
+    // (a count that does not divide ny was meant for blocks: one segment)
+    a.nseg = s->ny % s->nseg ? 1 : s->nseg;
+    a.wy = s->ny / a.nseg;
+    a.nchunks = (a.wy + s->chunk - 1) / s->chunk;  // the last chunk may be partial
+    a.seg_unit = a.wy;
+    a.seg_units = a.nseg;
     a.its = s->its;
     a.gts_base = gts0 - 1;
     a.xface = s->xface;
@@ -1106,8 +975,7 @@ int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
             cO += rg * cm;
         }
         const double u = (double)a.nb;
-        const size_t psm = K.fast ? (s->bs == 16 ? heat_fast_smem<16>(s->H) : heat_fast_smem<32>(s->H))
-                                  : stream_smem(s);
+        const size_t psm = stream_smem(s);
         // P, then Y on `stream` beside G on the side stream (G reads nothing
         // that Y writes: its valid cells depend on the prisms' faces only,
         // and adjacent bands share their segment boundaries, so G's
@@ -1851,7 +1719,6 @@ struct ps_batch {
     int device = 0, eq = 0, nv = 1, ops = 1, its = 1, bs = 0, mpss = 0, H = 0;
     int chunk = 32;  // column chunk of the generic streams (32 or 64)
     bool fast = false;
-    bool faces = false;  // Euler streams share faces (scratch beside the tile)
     cudaStream_t stream = nullptr;
     // the gap stream runs beside the y-bridge on a high-priority side stream
     cudaStream_t side = nullptr;
@@ -1873,6 +1740,8 @@ struct ps_batch {
     // unit) pairs per block size in use
     BlockInst* d_binst = nullptr;
     bool binst_current = false;
+    // Euler level by level: the instances with their level counters
+    MarchInst* d_minst = nullptr;
     struct Table {
         int vw, vh, n;
         int2* d;
@@ -1945,9 +1814,9 @@ int batch_upload(ps_batch* b)
             a.nb = I.nb;
             a.nseg = I.nseg;
             a.wy = I.ny / I.nseg;
-            a.nchunks = b->fast ? a.wy / kFastChunk : (a.wy + b->chunk - 1) / b->chunk;
-            a.seg_unit = b->fast ? 32 : a.wy;
-            a.seg_units = b->fast ? I.ny / 32 : I.nseg;
+            a.nchunks = (a.wy + b->chunk - 1) / b->chunk;
+            a.seg_unit = a.wy;
+            a.seg_units = I.nseg;
             a.off = par ? b->bs / 2 : 0;  // prism bands alternate by half a block
             a.its = b->its;
             a.gts_base = (int)I.level;
@@ -1983,8 +1852,7 @@ size_t batch_tile_smem(const ps_batch* b)
 
 size_t batch_stream_smem(const ps_batch* b)
 {
-    return batch_tile_smem(b) +
-           (b->faces ? sizeof(double) * euler_level_scratch(b->bs, b->chunk) : 0);
+    return batch_tile_smem(b);
 }
 
 size_t batch_seam_smem(const ps_batch* b)
@@ -2051,8 +1919,7 @@ bool batch_pick(int eq, int ops, int its, int chunk, HalfFn* half, PrepFn* prep)
     PS_BSET(PS_EQ_HEAT, 1, 1, 32, Heat)
     PS_BSET(PS_EQ_HEAT, 1, 2, 32, Heat)
     PS_BSET(PS_EQ_EULER, 2, 2, 32, Euler)
-    PS_BSET(PS_EQ_EULER_CELL, 2, 2, 32, EulerCell)
-    PS_BSET(PS_EQ_EULER_CELL, 2, 2, 64, EulerCell)
+    PS_BSET(PS_EQ_EULER, 2, 2, 64, Euler)
     PS_BSET(PS_EQ_HALF, 1, 2, 32, Half)
 #undef PS_BSET
     return false;
@@ -2164,6 +2031,66 @@ int batch_block_enqueue(ps_batch* b, const std::vector<BlockStep>& steps)
     return PS_OK;
 }
 
+// ---- Euler level by level ----
+bool batch_marches(const ps_batch* b)
+{
+    if (b->eq != PS_EQ_EULER) return false;
+    for (const auto& I : b->inst)
+        if (!march_constants(make_params_g(b->eq, I.globals))) return false;
+    return true;
+}
+
+int batch_march_upload(ps_batch* b)
+{
+    std::vector<MarchInst> d;
+    for (const auto& I : b->inst) {
+        const EqParams p = make_params_g(b->eq, I.globals);
+        d.push_back({{I.base[0], I.base[1]}, p.d[0], p.d[1], p.d[2], p.d[3], I.nx, I.ny, (int)I.level});
+    }
+    PSB_CUDA(b, cudaMemcpyAsync(b->d_minst, d.data(), d.size() * sizeof(MarchInst),
+                                cudaMemcpyHostToDevice, b->stream));
+    PSB_CUDA(b, cudaStreamSynchronize(b->stream));
+    b->desc_level.clear();
+    for (const auto& I : b->inst) b->desc_level.push_back(I.level);
+    return PS_OK;
+}
+
+// Rows of the strips, and their table.
+int batch_march_plan(ps_batch* b, int* hs, int* table)
+{
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
+    std::vector<BlockGrid> gs;
+    for (const auto& I : b->inst) gs.push_back({I.nx, I.ny});
+    *hs = march_rows(BlockGrids{gs.data(), (int)gs.size()}, sms);
+    return batch_table(b, kMarchW, *hs, table);
+}
+
+int batch_march_enqueue(ps_batch* b, int64_t nlevels, int hs, int table)
+{
+    const ps_batch::Table& t = b->tables[table];
+    int older = 2 * b->cur, newest = older + 1;  // as in run_levels
+    for (int64_t L = 1; L <= nlevels; ++L) {
+        const int next = (newest + 1) % 4;
+        launch_after(euler_march_batch, t.n, 32, 0, b->stream, (const MarchInst*)b->d_minst,
+                     (const int2*)t.d, newest, older, next, hs, (int)L);
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return bfail(b, PS_ERR_CUDA, "batched launch: %s", cudaGetErrorString(e));
+        older = newest;
+        newest = next;
+    }
+    if (newest % 2 == 0)
+        for (auto& I : b->inst) {
+            const size_t fe = (size_t)4 * I.nx * I.ny;
+            auto slot = [&](int q) { return I.base[q / 2] + (size_t)(q % 2) * fe; };
+            PSB_CUDA(b, cudaMemcpyAsync(slot(newest + 1), slot(newest), fe * sizeof(double),
+                                        cudaMemcpyDeviceToDevice, b->stream));
+            PSB_CUDA(b, cudaMemcpyAsync(slot(newest), slot(older), fe * sizeof(double),
+                                        cudaMemcpyDeviceToDevice, b->stream));
+        }
+    return PS_OK;
+}
+
 // Enqueue a whole run of nlevels levels, starting from parity b->cur.
 int batch_enqueue(ps_batch* b, int64_t nlevels, HalfFn half, int64_t* nlaunch)
 {
@@ -2224,13 +2151,10 @@ int ps_batch_create(ps_batch** out, int device, int equation, int count, const i
     b->mpss = blocksize / (2 * ops) - 1;
     b->H = default_levels(equation, its, blocksize, b->mpss);
     b->fast = equation == PS_EQ_HEAT && its == 1 && (blocksize == 16 || blocksize == 32);
-    // Euler: 64-column chunks where the tile fits, faces shared between cells
-    // where tile and scratch leave room for two CTAs per SM (as for a solver)
+    // Euler: 64-column chunks where the tile fits (as for a solver)
     if (!b->fast && equation == PS_EQ_EULER) {
         b->chunk = 64;
         if (batch_tile_smem(b) > 227 * 1024) b->chunk = 32;
-        b->faces = batch_tile_smem(b) + sizeof(double) * euler_level_scratch(b->bs, b->chunk) <=
-                   kFaceSmemCap;
     }
     int rc = PS_OK;
     std::vector<int2> units;
@@ -2253,7 +2177,7 @@ int ps_batch_create(ps_batch** out, int device, int equation, int count, const i
         // hold a chunk, so that the units of large and small instances take
         // similar times (a phase waits for its slowest unit)
         if (b->fast) {
-            I.nseg = std::max(1, I.ny / (8 * kFastChunk));
+            I.nseg = std::max(1, I.ny / 512);
         } else {
             const int minw = std::max(b->chunk, 2 * ops * (b->H + 1));
             I.nseg = 1;
@@ -2296,14 +2220,15 @@ int ps_batch_create(ps_batch** out, int device, int equation, int count, const i
         cudaError_t e = cudaMalloc(&b->d_desc, 4 * b->inst.size() * sizeof(SweptArgs));
         if (e == cudaSuccess && b->fast)
             e = cudaMalloc(&b->d_binst, b->inst.size() * sizeof(BlockInst));
+        if (e == cudaSuccess && equation == PS_EQ_EULER)
+            e = cudaMalloc(&b->d_minst, b->inst.size() * sizeof(MarchInst));
         if (e == cudaSuccess) e = cudaMalloc(&b->d_units, units.size() * sizeof(int2));
         if (e == cudaSuccess)
             e = cudaMemcpy(b->d_units, units.data(), units.size() * sizeof(int2), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) rc = bfail(b, PS_ERR_NOMEM, "batch tables: %s", cudaGetErrorString(e));
     }
     // the kernels of the chosen chunk width (prep opts them into large shared memory)
-    const int keq = (equation == PS_EQ_EULER && !b->faces) ? PS_EQ_EULER_CELL : equation;
-    if (rc == PS_OK && !batch_pick(keq, ops, its, b->chunk, &half, &prep))
+    if (rc == PS_OK && !batch_pick(equation, ops, its, b->chunk, &half, &prep))
         rc = bfail(b, PS_ERR_UNSUPPORTED, "no batched kernels for chunk %d", b->chunk);
     if (rc == PS_OK) prep();
     if (rc != PS_OK) {
@@ -2328,6 +2253,7 @@ int ps_batch_destroy(ps_batch* b)
         if (I.yface) cudaFree(I.yface);
     }
     if (b->d_binst) cudaFree(b->d_binst);
+    if (b->d_minst) cudaFree(b->d_minst);
     for (auto& t : b->tables) cudaFree(t.d);
     if (b->d_desc) cudaFree(b->d_desc);
     if (b->d_units) cudaFree(b->d_units);
@@ -2384,8 +2310,7 @@ int ps_batch_run(ps_batch* b, int64_t nlevels, int use_graph)
     PSB_CUDA(b, cudaSetDevice(b->device));
     HalfFn half;
     PrepFn prep;
-    batch_pick((b->eq == PS_EQ_EULER && !b->faces) ? PS_EQ_EULER_CELL : b->eq, b->ops, b->its,
-               b->chunk, &half, &prep);
+    batch_pick(b->eq, b->ops, b->its, b->chunk, &half, &prep);
     int64_t nsteps = (nlevels + b->H - 1) / b->H;  // half-cycles, or block launches
     std::vector<BlockStep> steps;
     const bool rebuild = !use_graph || !b->gexec || b->graph_levels != nlevels || b->graph_cur != b->cur;
@@ -2396,8 +2321,21 @@ int ps_batch_run(ps_batch* b, int64_t nlevels, int use_graph)
     } else if (b->fast) {
         nsteps = b->graph_launches;
     }
-    auto upload = [&]() -> int { return b->fast ? batch_block_upload(b) : batch_upload(b); };
+    // Euler: base buffers of two levels each, one launch per level
+    const bool march = batch_marches(b);
+    int hs = 0, table = 0;
+    if (march) {
+        nsteps = (nlevels + 1) / 2;  // (the newest level's base buffer changes every other level)
+        if (int rc = batch_march_plan(b, &hs, &table)) return rc;
+    }
+    auto upload = [&]() -> int {
+        return b->fast ? batch_block_upload(b) : (march ? batch_march_upload(b) : batch_upload(b));
+    };
     auto enqueue = [&](int64_t* n) -> int {
+        if (march) {
+            *n = nlevels;
+            return batch_march_enqueue(b, nlevels, hs, table);
+        }
         if (!b->fast) return batch_enqueue(b, nlevels, half, n);
         *n = (int64_t)steps.size();
         return batch_block_enqueue(b, steps);
@@ -2430,7 +2368,7 @@ int ps_batch_run(ps_batch* b, int64_t nlevels, int use_graph)
             b->graph_cur = b->cur;
             b->graph_launches = n;
         } else if (!b->fast && !batch_desc_current(b)) {
-            int rc = batch_upload(b);  // new level counters for the same graph
+            int rc = upload();  // new level counters for the same graph
             if (rc) return rc;
         }
         PSB_CUDA(b, cudaGraphLaunch(b->gexec, b->stream));

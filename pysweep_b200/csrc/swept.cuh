@@ -224,17 +224,6 @@ __host__ __device__ __forceinline__ int slot_count(int hmax)
     return LINEAR ? hmax + 2 : ITS + 1;
 }
 
-// Equations whose functor evaluates a whole stream level at once (faces
-// shared between cells): Eq::kFaceLevel and Eq::level<NT>.
-template <class Eq, class = void>
-struct FaceLevel {
-    static constexpr bool value = false;
-};
-template <class Eq>
-struct FaceLevel<Eq, decltype((void)Eq::kFaceLevel)> {
-    static constexpr bool value = Eq::kFaceLevel;
-};
-
 // ---------------------------------------------------------------- stream ----
 // One CTA = one (band, segment) block.  GAP = false: prism (UpPyramid);
 // GAP = true: gap (XBridge) centred on the band's upper boundary row.
@@ -330,12 +319,7 @@ __device__ __forceinline__ void stream_body(const SweptArgs& a, const int unit, 
                 cp_async_commit();
             }
             // compute level m
-            if constexpr (FaceLevel<Eq>::value) {
-                // faces shared between the cells of the level (scratch after the carry)
-                Eq::template level<NT>(cur, prv, out, rlo, rhi, (klo > O2 ? klo : O2) - OPS,
-                                       RC - OPS, RS, BX, gts, a.p,
-                                       carry + (size_t)(a.Hmax + 1) * CS, tid);
-            } else {
+            {
                 const int k = O2 + tk;
                 if (k >= klo && k < RC) {
                     // grid column of tile column k at level m (equations that

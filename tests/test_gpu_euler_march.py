@@ -98,3 +98,23 @@ def test_march_frames_at_any_address(off):
     got = _solve(ic, nl, 16, "swept", frames=fr)
     want, _, _ = oracle.standard("euler", ic, G, 2, nl, euler_square="mul")
     assert _same(fr.cpu().numpy(), want[1:]) and _same(got[0], want[-1])
+
+
+def test_batched_march_continues_and_mixes_stages():
+    """Instances of many sizes in one launch; an odd run, then one instance set
+    anew (its stages then alternate against the others'), then another run."""
+    from pysweep_b200 import Batch, plugin_constants
+    sizes = [(16, 16), (32, 64), (48, 128), (64, 16)]
+    ics = [_field("vortex", *s) for s in sizes]
+    with Batch("euler", sizes, its=2, blocksize=16) as b:
+        for i in range(len(sizes)):
+            b.set_constants(i, plugin_constants("euler", G))
+            b.set_state(i, ics[i])
+        b.run(5)
+        b.set_state(1, ics[1])
+        b.run(4)
+        b.run(4)
+        got = [(b.get_state(i, 0), b.get_state(i, 1)) for i in range(len(sizes))]
+    for i, (a, older) in enumerate(got):
+        ref = _solve(ics[i], 8 if i == 1 else 13, 16, "standard", threads=256)
+        assert _same(a, ref[0]) and _same(older, ref[1])
