@@ -17,9 +17,11 @@
 // and one of them needs no value but whether it exceeds 1e6 (limiters).  Every
 // result is the correctly rounded one, so levels equal the per-cell step's
 // (Euler::step) bitwise.  909 warp instructions per cell for the 1806 of tiles
-// with their faces in shared memory; G cells/s, tiles / here: 480² 6.6 / 9.3,
-// 1120² 8.8 / 16.0, 4096² 9.2 / 18.7.
+// with their faces in shared memory; G cells/s, tiles / here: 480² 6.6 / 11.4,
+// 1120² 8.8 / 18.7, 4096² 9.2 / 21.4.
 #pragma once
+#include <cmath>
+
 #include "equations.cuh"
 #include "heat_block.cuh"
 
@@ -458,16 +460,43 @@ __global__ void __launch_bounds__(32, kMarchWarps)
     march_body(a, u.y, sh);
 }
 
-// Rows of a strip: one wave of warps.
+// Rows of a strip: the fewest that fit one wave of warps, or 6 to 24 in several
+// waves where those cost less.  A strip costs its rows and 0.6 more (a grid's
+// last strips have what rows are left); of w waves, those after the first cost
+// 0.92 each (strips that start one after the other read the field in order:
+// 4096², G cells/s with strips of 164 rows 18.5, 48 20.8, 20 21.4, 6 20.0), and
+// the last 0.55 more the emptier it is (1600², w = 1.02 15.4, w = 1 18.5).  Over
+// grids of 480² to 4096² within 4% of the best strip.
 inline int march_rows(const BlockGrids& g, int sms)
 {
+    constexpr double start = 0.6, later = 0.92, drain = 0.55;
+    const double wave = (double)kMarchWarps * sms;
+    auto cost = [&](int hs) {
+        double w = 0.0;
+        for (int i = 0; i < g.n; ++i) {
+            const int rest = g.g[i].nx % hs;
+            w += ((g.g[i].ny + kMarchW - 1) / kMarchW) *
+                 (g.g[i].nx / hs + (rest ? (rest + start) / (hs + start) : 0.0)) / wave;
+        }
+        const double full = std::floor(w);
+        const double tail = w > full && full >= 1.0 ? drain * (1.0 - (w - full)) / full : 0.0;
+        return (hs + start) * (1.0 + later * std::max(0.0, w - 1.0) + tail);
+    };
     int lo = 1, hi = g.rows();
     while (lo < hi) {
         const int mid = (lo + hi) / 2;
-        if (g.blocks(kMarchW, mid) <= (long long)kMarchWarps * sms) hi = mid;
+        if ((double)g.blocks(kMarchW, mid) <= wave) hi = mid;
         else lo = mid + 1;
     }
-    return lo;
+    int best = lo;
+    // (a count of strips that no height brings into one wave costs its waves)
+    double least = g.blocks(kMarchW, lo) <= wave ? lo + start : cost(lo);
+    for (int hs = 6; hs <= std::min(24, lo - 1); ++hs)
+        if (cost(hs) < least) {
+            least = cost(hs);
+            best = hs;
+        }
+    return best;
 }
 
 // The constants for which the safe ranges above hold.
