@@ -473,9 +473,11 @@ struct BlockGrids {
 };
 
 // A tile's work relative to plain heat's: FP64 pipe time of a level, bytes of a
-// tile, latency of a level.
+// tile, latency of a level.  two: a level of tiles of two columns and eight rows,
+// whose warps exchange more per cell (1280²: 2.17 us per level where six rows of
+// four columns take 1.96; without it they were planned at 1.95 and 1.98).
 struct TileCost {
-    double level = 1.0, bytes = 1.0, latency = 1.0;
+    double level = 1.0, bytes = 1.0, latency = 1.0, two = 1.1;
 };
 
 // Estimated microseconds of one launch of T levels in tiles of shape t, or 0
@@ -492,7 +494,7 @@ inline double tile_us(const TileShape& t, int T, const BlockGrids& g, int sms,
     const double n = (double)((g.blocks(vw, vh) + sms - 1) / sms);  // tiles of the busiest SM
     const int occ = t.maxw / t.nw;
     const double k = std::min(n, (double)occ), rounds = std::max(1.0, n / occ);
-    const double level = 4.0 * t.nw * t.R * t.C / 1965.0 * 1.04 * c.level;
+    const double level = 4.0 * t.nw * t.R * t.C / 1965.0 * 1.04 * c.level * (t.C == 2 && t.R == 8 ? c.two : 1.0);
     const double kb = k * t.nw * t.R * t.C * 32 * 8 / 1024.0 * 0.03 * c.bytes;
     const double lat = (k * t.nw <= 12 ? 0.08 : 0.03) * c.latency;
     return 1.0 + n * T * level + (occ == 1 ? rounds : 1.0) * kb + (n - k) * 0.4 + lat * T * rounds;

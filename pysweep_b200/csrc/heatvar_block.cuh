@@ -290,8 +290,8 @@ constexpr TileShape kTilesAdj[] = {{2, 6, 16, 16}, {2, 6, 12, 16}, {2, 6, 8, 16}
 template <int ROLE>
 constexpr TileCost var_cost()
 {
-    return ROLE == VAR_FORWARD ? TileCost{1.0, 1.5, 1.5}
-                               : (ROLE == VAR_RECOMPUTE ? TileCost{1.8, 2.0, 1.5} : TileCost{1.6, 3.0, 1.5});
+    return ROLE == VAR_FORWARD ? TileCost{1.0, 1.5, 1.5, 1.0}
+                               : (ROLE == VAR_RECOMPUTE ? TileCost{1.8, 2.0, 1.5, 1.0} : TileCost{1.6, 3.0, 1.5, 1.0});
 }
 
 template <int ROLE>
