@@ -9,15 +9,15 @@
 //     lambda_n = lambda_{n+1} + L (C .* lambda_{n+1})
 //     dJ/dC   += lambda_{n+1} .* (L u_n),        dJ/dalpha = dJ/dC * dt/dx/dx
 // The forward stores u every `every` steps; the backward pass walks the
-// segments from the last to the first, recomputes the Laplacians of the
-// segment's states from its checkpoint into a work buffer, then runs the
-// adjoint steps backward through the segment.
+// segments from the last to the first, steps a segment's state forward from its
+// checkpoint, keeping it every few levels in a work buffer, then runs the
+// adjoint backward through the segment, those few levels per launch.
 //
 // The levels run in overlapped tiles, several per launch (heatvar_block.cuh):
-// the forward steps between checkpoints, the recompute of a segment, which
-// stores the Laplacians of its levels instead of the states, and the adjoint
-// levels, which read them.  Every cell sees the one-step operations in their
-// order, so the number of levels per launch changes no bit.
+// the forward steps, and the adjoint levels, whose tile recomputes the levels'
+// Laplacians on chip.  ps_heatvar_recompute stores a segment's Laplacians for
+// the adjoint solvers, which read them.  Every cell sees the one-step operations
+// in their order, so the number of levels per launch changes no bit.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -214,9 +214,16 @@ extern "C" int ps_heatvar_adjoint(const double* d_courant, const double* d_check
     const int sms = sm_count();
     const int64_t nseg = (nsteps + every - 1) / every;
     auto length = [&](int64_t k) { return (int)(std::min<int64_t>((k + 1) * every, nsteps) - k * every); };
+    const BlockGrid grid{nx, ny};
+    auto cut = [&](int n) {  // levels of each launch of a segment of n
+        std::vector<int> t;
+        const BlockPlan plan = plan_back(BlockGrids{&grid, 1}, n, sms);
+        for (int done = 0; done < n; done += t.back()) t.push_back(plan_next(plan, n - done, 1));
+        return t;
+    };
     // every segment but the last has `every` steps
-    const std::vector<int> whole = launches<VAR_LAMBDA>(every, nx, ny, sms);
-    const std::vector<int> tail = launches<VAR_LAMBDA>(nseg ? length(nseg - 1) : 0, nx, ny, sms);
+    const std::vector<int> whole = cut((int)std::min<int64_t>(every, nsteps));
+    const std::vector<int> tail = cut(nseg ? length(nseg - 1) : 0);
     const int64_t count = nseg ? (int64_t)tail.size() + (nseg - 1) * (int64_t)whole.size() : 0;
     if ((rc = adj_cuda(cudaMemsetAsync(d_galpha, 0, n * sizeof(double), st), err, errlen))) return rc;
     // lambda ping-pong between d_lam0 and d_lamwork, arranged so that lambda_0
@@ -225,28 +232,29 @@ extern "C" int ps_heatvar_adjoint(const double* d_courant, const double* d_check
     if ((rc = adj_cuda(cudaMemcpyAsync(lam, d_lamT, n * sizeof(double), cudaMemcpyDeviceToDevice, st),
                        err, errlen)))
         return rc;
-    VarArgs a = var_args(d_courant, nx, ny);
-    a.step = -(long long)n;
+    BackArgs a;
+    memset(&a, 0, sizeof a);
+    a.C = d_courant;
     a.g = d_galpha;
+    a.nx = nx;
+    a.ny = ny;
+    VarArgs f = var_args(d_courant, nx, ny);
     for (int64_t k = nseg - 1; k >= 0; --k) {
-        const int len = length(k);
-        // L(u_n) of the segment's levels into d_states.  Scratch for the states
-        // between launches: lambda's other buffer, which the launch before the
-        // last leaves its state in, and the last level's own slot, which only
-        // the last launch writes
-        double* other = lam == d_lam0 ? d_lamwork : d_lam0;
-        recompute(d_courant, d_checkpoints + (size_t)k * n, d_states, len, nx, ny, other,
-                  d_states + (size_t)(len - 1) * n, sms, st);
-        // adjoint levels len-1 .. 0 of the segment
-        int done = 0;
-        for (int T : k == nseg - 1 ? tail : whole) {
-            double* out = lam == d_lam0 ? d_lamwork : d_lam0;
+        const std::vector<int>& t = k == nseg - 1 ? tail : whole;
+        const double* u0 = d_checkpoints + (size_t)k * n;
+        // the state every launch but the first starts from: d_states[0], [1], ..
+        f.in = u0;
+        for (size_t j = 0; j + 1 < t.size(); ++j) {
+            f.out = d_states + j * n;
+            launch_var<VAR_FORWARD>(f, t[j], sms, st);
+            f.in = f.out;
+        }
+        for (size_t j = t.size(); j-- > 0;) {
+            a.u = j ? d_states + (j - 1) * n : u0;
             a.in = lam;
-            a.out = out;
-            a.lap = d_states + (size_t)(len - 1 - done) * n;
-            launch_var<VAR_LAMBDA>(a, T, sms, st);
-            lam = out;
-            done += T;
+            lam = lam == d_lam0 ? d_lamwork : d_lam0;
+            a.out = lam;
+            launch_back(a, t[j], sms, st);
         }
     }
     scale_kernel<<<1024, 256, 0, st>>>(d_galpha, n, dt / dx / dx);

@@ -326,4 +326,235 @@ void launch_var(VarArgs a, int T, int sms, cudaStream_t st)
         launch_after(heatvar_tile<ROLE, 2, ADJ ? 6 : 8, 16>, units, 32 * t.nw, smem, st, a);
 }
 
+// --------------------------------------------------------------- backward --
+// T levels of a checkpoint segment backward in one launch: a tile steps the
+// state the levels start from forward once more, keeping its exact cells'
+// Laplacians in shared memory, then lambda backward through them, so that they
+// never reach global memory.
+//
+// What bounds it: the two passes one after the other, 17 FP64 operations per
+// cell and level on cells of which a quarter is halo, and 48 bytes per cell and
+// launch; at most 227 KB of Laplacians on an SM.  Two CTAs or more per SM: with
+// one, its loads and stores hide behind nothing (2048², T = 4, 8 warps of 6 rows
+// twice 15.2, 16 warps once 21.9 us per level).  us per level, recompute +
+// adjoint by themselves / here with the forward steps that lead to the levels'
+// start: 256² 2.08 / 1.49, 512² 2.67 / 2.52, 1024 x 1536 9.4 / 8.5, 2048² 26.6 / 20.9,
+// 4096² 96 / 77.
+struct BackArgs {
+    const double* u;    // the state before the levels
+    const double* C;
+    const double* in;   // lambda after them
+    double* out;        // and before them
+    double* g;          // sums, updated in place
+    int nx, ny, T, ncs, vw, vh;
+};
+
+// Shared memory: the outer rows, then Laplacians [level][exact row][lane][2].
+__host__ __device__ constexpr size_t back_smem(int R, int nw, int T)
+{
+    return tile_smem<2>(nw) + sizeof(double) * 64 * T * (nw * R - 2 * T);
+}
+
+// MAXW warps per CTA, two such CTAs on an SM.
+template <int R, int MAXW>
+__global__ void __launch_bounds__(32 * MAXW, 2) heatvar_back(const __grid_constant__ BackArgs a)
+{
+    extern __shared__ __align__(16) double tile_sm[];
+    constexpr int C = 2;
+    const int nw = blockDim.x >> 5, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int nx = a.nx, ny = a.ny, T = a.T;
+    const int cs = blockIdx.x % a.ncs, rs = blockIdx.x / a.ncs;
+    const int rlo = rs * a.vh, rhi = min(rlo + a.vh, nx);  // exact rows
+    const int clo = cs * a.vw, chi = min(clo + a.vw, ny);  // exact columns
+    const int c0 = clo - tile_halo<C>(T) + C * lane;
+    const int r0 = rlo - T + w * R;
+    const int gcol = wrap(c0, ny);
+    const bool ok = c0 >= clo && c0 < chi;
+    const int ne = nw * R - 2 * T;  // exact rows of a whole tile
+    double* lap = tile_sm + 32 * C * nw * 4 + lane * 2;
+    // where level m's Laplacian of the warp's row i lies; rows that are exact
+    auto lap_at = [&](int m, int i) { return lap + ((m - 1) * ne + w * R + i - T) * 64; };
+    auto kept = [&](int i) { return w * R + i >= T && w * R + i < T + ne; };
+    auto mine = [&](int i) { return r0 + i >= rlo && r0 + i < rhi && ok; };
+    auto slot = [&](int buf, int ww, int b) {
+        return tile_sm + ((buf * nw + ww) * 2 + b) * (32 * C) + lane * 2;
+    };
+    auto put = [&](int buf, int b, const double (&v)[C]) {
+        *reinterpret_cast<double2*>(slot(buf, w, b)) = make_double2(v[0], v[1]);
+    };
+    auto get = [&](int buf, int ww, int b, double (&v)[C]) {
+        const double2 x = *reinterpret_cast<const double2*>(slot(buf, ww, b));
+        v[0] = x.x;
+        v[1] = x.y;
+    };
+    auto load = [&](const double* p, double (&v)[C]) {
+        const double2 x = *reinterpret_cast<const double2*>(p);
+        v[0] = x.x;
+        v[1] = x.y;
+    };
+    const int wu = w == 0 ? 0 : w - 1, wd = w == nw - 1 ? w : w + 1;
+    double cr[R][C], u[R][C], m0[C], m1[C], m2[C], l[C];
+    grid_wait();
+    {
+        int r = wrap(r0, nx);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const size_t o = (size_t)r * ny + gcol;
+            load(a.u + o, u[i]);
+            load(a.C + o, cr[i]);
+            r = r + 1 == nx ? 0 : r + 1;
+        }
+    }
+    grid_release();
+    put(0, 0, u[0]);
+    put(0, 1, u[R - 1]);
+    __syncthreads();
+    // the states u_n .. : rows in ascending order, the old row above kept aside
+    for (int m = 1; m <= T; ++m) {
+        const int b = (m - 1) & 1;
+        get(b, wu, 1, m0);
+        get(b, wd, 0, m2);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            double old[C];
+#pragma unroll
+            for (int j = 0; j < C; ++j) old[j] = u[i][j];
+            if (i < R - 1) var_row<C>(m0, old, u[i + 1], cr[i], u[i], l);
+            else var_row<C>(m0, old, m2, cr[i], u[i], l);
+            if (kept(i)) *reinterpret_cast<double2*>(lap_at(m, i)) = make_double2(l[0], l[1]);
+#pragma unroll
+            for (int j = 0; j < C; ++j) m0[j] = old[j];
+            if (i == 0) put(1 - b, 0, u[0]);
+        }
+        put(1 - b, 1, u[R - 1]);
+        __syncthreads();
+    }
+    // lambda backward: u now holds it
+    double g[R][C];
+    {
+        int r = wrap(r0, nx);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const size_t o = (size_t)r * ny + gcol;
+            load(a.in + o, u[i]);
+            g[i][0] = g[i][1] = 0.0;
+            if (mine(i)) load(a.g + (size_t)(r0 + i) * ny + c0, g[i]);
+            r = r + 1 == nx ? 0 : r + 1;
+        }
+    }
+    // exchanged, and differenced
+    auto operand = [&](int i, double (&m)[C]) {
+#pragma unroll
+        for (int j = 0; j < C; ++j) m[j] = __dmul_rn(cr[i][j], u[i][j]);
+    };
+    operand(0, m0);
+    put(0, 0, m0);
+    operand(R - 1, m0);
+    put(0, 1, m0);
+    __syncthreads();
+    for (int m = T; m >= 1; --m) {
+        const int b = (T - m) & 1;
+        get(b, wu, 1, m0);
+        operand(0, m1);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            if (i < R - 1) operand(i + 1, m2);
+            else get(b, wd, 0, m2);
+            if (kept(i)) {
+                load(lap_at(m, i), l);
+#pragma unroll
+                for (int j = 0; j < C; ++j) g[i][j] = __fma_rn(u[i][j], l[j], g[i][j]);
+            }
+            const double left = __shfl_up_sync(0xffffffffu, m1[1], 1);
+            const double right = __shfl_down_sync(0xffffffffu, m1[0], 1);
+            const double ym[C] = {left, m1[0]}, yp[C] = {m1[1], right};
+#pragma unroll
+            for (int j = 0; j < C; ++j) {
+                const double lm = __dadd_rn(__dadd_rn(__fma_rn(-2.0, m1[j], m2[j]), m0[j]),
+                                            __dadd_rn(__fma_rn(-2.0, m1[j], yp[j]), ym[j]));
+                u[i][j] = __dadd_rn(u[i][j], lm);
+            }
+            if (i == 0 || i == R - 1) {
+                double q[C];
+                operand(i, q);
+                put(1 - b, i == 0 ? 0 : 1, q);
+            }
+#pragma unroll
+            for (int j = 0; j < C; ++j) {
+                m0[j] = m1[j];
+                m1[j] = m2[j];
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+        if (mine(i)) {
+            const size_t o = (size_t)(r0 + i) * ny + c0;
+            *reinterpret_cast<double2*>(a.out + o) = make_double2(u[i][0], u[i][1]);
+            *reinterpret_cast<double2*>(a.g + o) = make_double2(g[i][0], g[i][1]);
+        }
+}
+
+// The tiles that are built: six rows per warp and 8 warps twice on an SM, four
+// rows and 10 warps.
+constexpr int kBackMaxT = 8;
+constexpr TileShape kTilesBack[] = {{2, 6, 8, 8}, {2, 6, 6, 8}, {2, 6, 4, 8},
+                                    {2, 4, 10, 10}, {2, 4, 8, 10}, {2, 4, 6, 10}};
+
+// Estimated microseconds of one launch (fitted to launches of 256² to 2048²,
+// within 30%), or 0 where no cell of the tile stays exact.
+inline double back_us(const TileShape& t, int T, const BlockGrids& g, int sms)
+{
+    const int vw = tile_vw(t, T), vh = tile_vh(t, T);
+    if (vw < 8 || vh < 2) return 0.0;
+    const int occ = std::min(2 * t.maxw / t.nw, (int)(227 * 1024 / (back_smem(t.R, t.nw, T) + 1024)));
+    if (occ < 1) return 0.0;
+    const double n = (double)((g.blocks(vw, vh) + sms - 1) / sms), rounds = std::max(1.0, n / occ);
+    return 1.24 + n * (0.0061 * T + 0.04) * t.nw * t.R + (0.39 * T + 0.38) * rounds;
+}
+
+inline TileShape best_back(int T, const BlockGrids& g, int sms, double* us)
+{
+    TileShape best = kTilesBack[0];
+    *us = 1e300;
+    for (const TileShape& t : kTilesBack) {
+        const double one = back_us(t, T, g, sms);
+        if (one > 0 && one < *us) {
+            *us = one;
+            best = t;
+        }
+    }
+    return best;
+}
+
+inline BlockPlan plan_back(const BlockGrids& g, int nlevels, int sms)
+{
+    BlockPlan best{false, 1, 1e300};
+    for (int T = 1; T <= kBackMaxT; ++T) {
+        const int k = (nlevels + T - 1) / T;
+        double one;
+        best_back(T, g, sms, &one);
+        if (k * one < best.us) best = BlockPlan{false, T, k * one};
+    }
+    return best;
+}
+
+// One launch of T levels; a: pointers, nx, ny.
+inline void launch_back(BackArgs a, int T, int sms, cudaStream_t st)
+{
+    const BlockGrid grid{a.nx, a.ny};
+    double us;
+    const TileShape t = best_back(T, BlockGrids{&grid, 1}, sms, &us);
+    a.T = T;
+    a.vw = tile_vw(t, T);
+    a.vh = tile_vh(t, T);
+    a.ncs = (a.ny + a.vw - 1) / a.vw;
+    const int units = a.ncs * ((a.nx + a.vh - 1) / a.vh);
+    const size_t smem = back_smem(t.R, t.nw, T);
+    auto k = t.R == 6 ? heatvar_back<6, 8> : heatvar_back<4, 10>;
+    allow_big_smem(k);
+    launch_after(k, units, 32 * t.nw, smem, st, a);
+}
+
 }  // namespace psb

@@ -53,6 +53,14 @@ def test_tiles_against_plain_torch(nx, ny, n, every):
     assert ((ga - galpha).abs() <= tol).all()
 
 
+@pytest.mark.parametrize("nx,ny,n,every", [(3, 64, 8, 8), (30, 64, 9, 9), (256, 320, 17, 17), (700, 768, 11, 6),
+                                           (1600, 1536, 9, 9), (2100, 2112, 7, 7)])
+def test_backward_tiles(nx, ny, n, every):
+    """Levels backward in one launch, in tiles of every shape: grids smaller than
+    a tile's halo, one over a tile, several tiles per SM."""
+    test_tiles_against_plain_torch(nx, ny, n, every)
+
+
 def test_recompute_stores_every_laplacian():
     import torch
     from pysweep_b200 import _lib
