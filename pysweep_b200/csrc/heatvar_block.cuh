@@ -336,10 +336,10 @@ void launch_var(VarArgs a, int T, int sms, cudaStream_t st)
 // cell and level on cells of which a quarter is halo, and 48 bytes per cell and
 // launch; at most 227 KB of Laplacians on an SM.  Two CTAs or more per SM: with
 // one, its loads and stores hide behind nothing (2048², T = 4, 8 warps of 6 rows
-// twice 15.2, 16 warps once 21.9 us per level).  us per level, recompute +
+// twice 14.4, 16 warps once 21.9 us per level).  us per level, recompute +
 // adjoint by themselves / here with the forward steps that lead to the levels'
-// start: 256² 2.08 / 1.49, 512² 2.67 / 2.52, 1024 x 1536 9.4 / 8.5, 2048² 26.6 / 20.9,
-// 4096² 96 / 77.
+// start: 256² 2.08 / 1.50, 512² 2.67 / 2.24, 1024 x 1536 9.4 / 8.25, 2048² 26.6 / 20.1,
+// 4096² 96 / 75.
 struct BackArgs {
     const double* u;    // the state before the levels
     const double* C;
@@ -460,11 +460,11 @@ __global__ void __launch_bounds__(32 * MAXW, 2) heatvar_back(const __grid_consta
         for (int i = 0; i < R; ++i) {
             if (i < R - 1) operand(i + 1, m2);
             else get(b, wd, 0, m2);
-            if (kept(i)) {
-                load(lap_at(m, i), l);
+            // (rows that are not exact take another row's: their sums go nowhere;
+            // without the branch the rows overlap: 2048² 15.2 -> 14.4)
+            load(lap + ((m - 1) * ne + min(max(w * R + i - T, 0), ne - 1)) * 64, l);
 #pragma unroll
-                for (int j = 0; j < C; ++j) g[i][j] = __fma_rn(u[i][j], l[j], g[i][j]);
-            }
+            for (int j = 0; j < C; ++j) g[i][j] = __fma_rn(u[i][j], l[j], g[i][j]);
             const double left = __shfl_up_sync(0xffffffffu, m1[1], 1);
             const double right = __shfl_down_sync(0xffffffffu, m1[0], 1);
             const double ym[C] = {left, m1[0]}, yp[C] = {m1[1], right};
