@@ -1,5 +1,7 @@
 // C ABI of the B200 swept space-time solver (declarations: include/pysweep_b200.h).
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cstdarg>
@@ -1182,6 +1184,27 @@ bool hook_encode(const void* value, size_t nbytes, size_t size, char kind, unsig
 
 }  // namespace
 
+// Maps the pages of a host buffer about to receive n bytes, in one call, while
+// the GPU may still be busy.  A fresh allocation otherwise takes a page fault
+// every 4 KB of the copy: 25 MB in 25 arrays, 10 ms by faults, 5 ms here, the copy
+// itself 2.  Looks at one page only where they are mapped already.  Advice: the
+// copy works whatever becomes of it.
+static void map_host_pages(void* p, size_t n)
+{
+#ifdef MADV_POPULATE_WRITE
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t lo = ((uintptr_t)p + page - 1) / page * page, hi = ((uintptr_t)p + n) / page * page;
+    if (hi < lo + 16 * page) return;
+    unsigned char there = 1;
+    const uintptr_t mid = (lo + (hi - lo) / 2) / page * page;
+    if (mincore((void*)mid, page, &there) == 0 && !(there & 1))
+        madvise((void*)lo, hi - lo, MADV_POPULATE_WRITE);
+#else
+    (void)p;
+    (void)n;
+#endif
+}
+
 extern "C" {
 
 const char* ps_version(void) { return kVersion; }
@@ -1599,6 +1622,7 @@ int ps_get_state(ps_solver* s, double* dst, int level, int dst_on_device)
     if (level < 0 || level >= s->its) return fail(s, PS_ERR_INVALID, "level %d not in [0, its)", level);
     PS_CUDA(s, cudaSetDevice(s->device));
     const size_t fe = field_elems(s);
+    if (!dst_on_device) map_host_pages(dst, nbytes(s, fe));
     PS_CUDA(s, cudaMemcpyAsync(dst, at(s, s->base[s->cur], (size_t)(s->its - 1 - level) * fe),
                                nbytes(s, fe),
                                dst_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
@@ -2386,6 +2410,7 @@ int ps_batch_get_state(ps_batch* b, int index, double* dst, int level, int dst_o
     PSB_CUDA(b, cudaSetDevice(b->device));
     BatchInst& I = b->inst[index];
     const size_t f = (size_t)b->nv * I.nx * I.ny;
+    if (!dst_on_device) map_host_pages(dst, f * sizeof(double));
     PSB_CUDA(b, cudaMemcpyAsync(dst, I.base[b->cur] + (size_t)(b->its - 1 - level) * f,
                                 f * sizeof(double),
                                 dst_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
