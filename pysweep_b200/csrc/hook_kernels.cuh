@@ -86,13 +86,16 @@ extern "C" __global__ void __launch_bounds__(128) psh_octahedron(SweptArgs a)
 // T levels of an overlapped block (T = 1: one level of the standard
 // decomposition, pysweep/core/pysweep.cu:259-275).  The tile's newest level (and
 // the one before it, where `older` is given) with a periodic halo of OPS cells
-// per level into shared memory; level m on the rows and columns that are still
-// exact, a warp to a row; the last level's exact cells back (two base levels: the
-// one before it, too), and every level that a frame keeps.  Level 1 spans
-// PSH_BLK_W columns, so that no warp's pass over a row runs nearly empty, and
-// the hook's work is the same on every level: bound by its shared-memory reads
-// (heat: five reads and a write for eight FP64 operations).  Heat as a hook,
-// 200 levels at 1024², prisms of blocksize 16 / here: 3.67 / 0.96 ms.
+// per level into shared memory, two columns per load where rows and addresses
+// allow; level m on the rows and columns that are still exact, a warp to a row;
+// the last level's exact cells back (two base levels: the one before it, too),
+// and every level that a frame keeps.  Level 1 spans PSH_BLK_W columns, so that
+// no warp's pass over a row runs nearly empty.
+// What bounds it: the hook's shared-memory reads (heat: five reads and a write
+// for eight FP64 operations), and the tile's way in and out: a hook that only
+// copies takes three quarters of heat's time.  Heat as a hook, 200 levels at
+// 1024²: prisms of blocksize 16 3.67 ms, here 0.85; with one column per load and
+// a division per row and variable 0.97.
 struct HookFrames {
     double* level[PSH_BLK_MAXT];
 };
@@ -104,51 +107,66 @@ extern "C" __global__ void __launch_bounds__(psb::kBlkNT)
 {
     using namespace psb;
     constexpr int OPS = PSH_OPS, NV = PSH_NV, CC = kBlkCols;
-    constexpr int NP = (CC + 31) / 32;  // passes of a warp over a row
-    extern __shared__ double t[];
+    extern __shared__ __align__(16) double t[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, NW = blockDim.x >> 5;
     const int RR = rows1 + 2 * OPS, SL = NV * RR * CC;  // tile rows, one slot
     const int ih = rows1 - 2 * OPS * (T - 1), iw = PSH_BLK_W - 2 * OPS * (T - 1);
     const int x0 = blockIdx.y * ih, y0 = blockIdx.x * iw;
     const size_t vs = (size_t)nx * ny;
-    int g[NP];  // grid columns of the lane's tile columns lane + 32 p
-#pragma unroll
-    for (int p = 0; p < NP; ++p) g[p] = wrap(y0 - OPS * T + lane + 32 * p, ny);
+    // two columns at once: tile and grid columns of one parity and rows of whole
+    // pairs (y0, CC and iw are even; a state is 16-byte aligned where its user's
+    // buffer is)
+    const bool pairs = ny % 2 == 0 && OPS * T % 2 == 0 &&
+                       (((size_t)newest | (size_t)older | (size_t)out | (size_t)out1) & 15) == 0;
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int e = w; e < NV * RR; e += NW) {
-        const int v = e / RR, i = e % RR;
-        const size_t o = v * vs + (size_t)wrap(x0 - OPS * T + i, nx) * ny;
+    auto load = [&](int i, int k, bool two) {  // tile row i, column k (and the next)
+        const size_t o = (size_t)wrap(x0 - OPS * T + i, nx) * ny + wrap(y0 - OPS * T + k, ny);
+        double* to = t + SL + i * CC + k;
 #pragma unroll
-        for (int p = 0; p < NP; ++p) {
-            const int k = lane + 32 * p;
-            if (k < CC) {
-                cp_async8(t + SL + e * CC + k, newest + o + g[p]);
-                if (older) cp_async8(t + e * CC + k, older + o + g[p]);
+        for (int v = 0; v < NV; ++v) {
+            double* q = to + v * RR * CC;
+            if (two) {
+                cp_async16(q, newest + v * vs + o);
+                if (older) cp_async16(q - SL, older + v * vs + o);
+            } else {
+                cp_async8(q, newest + v * vs + o);
+                if (older) cp_async8(q - SL, older + v * vs + o);
             }
         }
-    }
+    };
+    if (pairs)
+        for (int e = threadIdx.x; e < RR * (CC / 2); e += blockDim.x)
+            load(e / (CC / 2), e % (CC / 2) * 2, true);
+    else
+        for (int e = threadIdx.x; e < RR * CC; e += blockDim.x) load(e / CC, e % CC, false);
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // the exact cells of level m to global memory
-    auto store = [&](double* dst, int m) {
-        const double* src = t + (m + 1) * SL;
-        for (int e = w; e < NV * ih; e += NW) {
-            const int v = e / ih, i = e % ih;
-            if (x0 + i >= nx) continue;
-            double* row = dst + v * vs + (size_t)(x0 + i) * ny + y0;
-            const double* from = src + (v * RR + i + OPS * T) * CC + OPS * T;
-            for (int k = lane; k < iw && y0 + k < ny; k += 32) row[k] = from[k];
-        }
+    auto store = [&](double* dst, int m, bool two) {
+        const double* src = t + (m + 1) * SL + OPS * T * (CC + 1);
+        const int rows = min(ih, nx - x0), cols = min(iw, ny - y0);
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+            for (int i = w; i < rows; i += NW) {
+                double* row = dst + v * vs + (size_t)(x0 + i) * ny + y0;
+                const double* from = src + (v * RR + i) * CC;
+                if (two) {
+                    for (int k = 2 * lane; k < cols; k += 64)
+                        *reinterpret_cast<double2*>(row + k) = *reinterpret_cast<const double2*>(from + k);
+                } else {
+                    for (int k = lane; k < cols; k += 32) row[k] = from[k];
+                }
+            }
     };
     for (int m = 1; m <= T; ++m) {
         const int lo = OPS * m;
         for (int i = lo + w; i < RR - lo; i += NW)
             for (int k = lo + lane; k < CC - lo; k += 32) psh_std::step(t, m * SL + i * CC + k, gts + m - 1);
         __syncthreads();
-        if (any_frame && frames.level[m - 1]) store(frames.level[m - 1], m);
+        if (any_frame && frames.level[m - 1]) store(frames.level[m - 1], m, false);
     }
-    store(out, T);
-    if (out1) store(out1, T - 1);
+    store(out, T, pairs);
+    if (out1) store(out1, T - 1, pairs);
 }
