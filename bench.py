@@ -4,8 +4,8 @@
 Workload (one "step" = one full solve): the 2-D heat equation u_t = u_xx + u_yy
 on the periodic unit square, 8192 x 8192 FP64 cells, forward Euler with
 dt = 0.2*dx^2, 5000 time steps, swept decomposition with blocksize 32
-(12 levels per half-cycle, the library's default for this shape; at most
-15 fit a 32-row band).  The initial field is a seeded sum of 8 periodic
+(the library runs it in overlapped blocks of 8 levels per launch; its tiling
+reports 12 levels per half-cycle).  The initial field is a seeded sum of 8 periodic
 Fourier modes (amplitudes U(0,1)).  The 537 MB field is larger than the
 126 MB L2, so consecutive steps do not run from cache.
 
@@ -159,7 +159,7 @@ def max_sm_mhz(clk):
 
 
 def fp64_roof(cells, ms, clk):
-    """The swept streams are bound by FP64 issue, not HBM: FP64 instructions
+    """The swept blocks are bound by FP64 issue, not HBM: FP64 instructions
     per second of a kernel against the FP64 pipe's rate (64 lanes per SM) at
     the GPU's maximum SM clock (an FMA counts as one instruction), in
     T instructions/s.  The rate at the sampled median clock is reported
@@ -179,7 +179,7 @@ def fp64_roof(cells, ms, clk):
 
 
 def ncu_traffic(kind, n, bs, h):
-    """DRAM bytes per launch of one kernel kind (h levels per half-cycle)
+    """DRAM bytes per launch of one kernel kind (h: the tiling's levels)
     from the committed ncu profile summary (measured at this grid size, or
     scaled from a smaller capture where its header says so); None where the
     summary has no line for this size."""
@@ -263,8 +263,8 @@ def roofline(prof, cell_bytes, clk, traffic_key=None):
     """Roofline of the dominant kernel of a run, from the per-launch CUDA-event
     profile {kind: (ms, launches, cell updates)}.
 
-    The swept streams reuse every loaded value across the levels of a
-    half-cycle, so their binding resource is the FP64 pipe, not HBM: `bound`,
+    The swept blocks reuse every loaded value across the levels of a
+    launch, so their binding resource is the FP64 pipe, not HBM: `bound`,
     `achieved`, `peak` and `frac` are FP64 instructions per second against the
     pipe's rate at the maximum SM clock.  `effective_bytes` keeps the
     16-bytes-per-cell-update figure (a read and a write of each value) against

@@ -144,11 +144,13 @@ int ps_get_global_value(ps_solver *s, const char *name, double *value);
  * Tiling knobs of the swept decomposition (0 keeps the current value):
  * h = levels per half-cycle (1..MPSS), nseg = column blocks per row band,
  * chunk = streaming chunk width (32 or 64) of the generic streams,
- * threads = 128 (default: register-resident heat streams where they apply)
- * or 256 (always the generic shared-memory streams).
+ * threads = 128 (default: overlapped blocks for heat, its per-cell-courant
+ * forms and step hooks, Euler level by level) or 256 (always the shared-memory
+ * prisms and seams).  A configured h also bounds the levels that a block runs
+ * per launch.
  * The defaults reproduce the reference's bs-row bands with MPSS levels per
- * half-cycle, except heat with forward Euler at bs 32 (12 levels, measured
- * faster); results do not depend on the tiling.
+ * half-cycle, except heat with forward Euler at bs 32 (12 levels); results do
+ * not depend on the tiling.
  */
 int ps_configure(ps_solver *s, int h, int nseg, int chunk, int threads);
 
@@ -231,8 +233,8 @@ int ps_set_stream(ps_solver *s, void *stream);
  * Per-kernel device timing.  ps_profile(s, 1) resets the counters and brackets
  * every following launch with CUDA events on the solver's stream;
  * ps_profile_read returns, for one kernel kind (0 prism stream, 1 Y-bridge
- * seam, 2 gap stream, 3 octahedron seam, 4 standard step), the summed device
- * time in ms, the number of launches and the algorithmic cell updates those
+ * seam, 2 gap stream, 3 octahedron seam, 4 standard step, 5 overlapped block or
+ * level of a swept run), the summed device time in ms, the number of launches and the algorithmic cell updates those
  * launches performed.  Both synchronise the stream.  No reference
  * counterpart: the reference times whole runs only (pysweep/core/io.py:10-27).
  */
@@ -257,7 +259,8 @@ const char *ps_last_error(const ps_solver *s);
  * every temporary lives in one static device array of 128 MiB that each GPU
  * holds from library load to process exit.  Sizes whose scratch (one field plus
  * the prism faces, about 22*nx*ny bytes at blocksize 32) exceeds it are
- * rejected with PS_ERR_INVALID and a message in err.  The first call on a
+ * rejected with PS_ERR_INVALID and a message in err (the overlapped blocks that
+ * run now need the field only; the limit has stayed).  The first call on a
  * device resolves the array's device address, so make it before any stream
  * capture; that address is kept for the life of the process, so a
  * cudaDeviceReset after the first call is not supported.  Calls share the array: two calls that overlap on the GPU (other
@@ -274,16 +277,16 @@ int ps_heat_swept_noalloc(const double *d_in, double *d_out, int nx, int ny, int
  * Batches: many independent fields (uneven sizes, one equation, one blocksize)
  * advanced together.  No counterpart in the reference, which runs one field
  * per Solver; the per-instance equivalent is one ps_solver per field.  Every
- * phase of a half-cycle is one launch for all instances (a flat table of
- * (instance, band segment) units); with use_graph != 0 the launches of a whole
+ * overlapped block (heat, forward Euler), level (Euler) or phase of a half-cycle
+ * (the other equations) is one launch for all instances (a flat table of
+ * (instance, unit) pairs); with use_graph != 0 the launches of a whole
  * run are captured once into a CUDA graph and replayed.  Constants are per
  * instance (index) or for all (index = -1).  Each instance counts the levels
  * run since its state was set: the first level after ps_batch_set_state sees
  * globalTimeStep = 1 (pysweep/core/solver.py:162) and consecutive
  * ps_batch_run calls continue the count, so runs of any length (odd ones with
- * two stages included) add up to one run of their total.  Register streams (heat, forward
- * Euler, blocksize 16/32) need nx, ny multiples of 32; the other equations use
- * the shared-memory streams with one segment per band.
+ * two stages included) add up to one run of their total.  Heat with forward Euler
+ * at blocksize 16 or 32 needs nx, ny multiples of 32.
  */
 typedef struct ps_batch ps_batch;
 int ps_batch_create(ps_batch **out, int device, int equation, int count, const int *nx,
@@ -313,10 +316,11 @@ const char *ps_batch_last_error(const ps_batch *b);
  *
  * ps_heatvar_adjoint: for J(u_T) with d_lamT = dJ/du_T, writes dJ/du0 to
  * d_lam0 and dJ/dalpha to d_galpha, walking the checkpoint segments backward:
- * each segment's states are recomputed into d_states (every fields), then the
- * adjoint steps lambda_n = lambda_{n+1} + L(C .* lambda_{n+1}),
- * dJ/dC += lambda_{n+1} .* L u_n run backward through it.  d_lamwork is a
- * scratch field.  `err` receives a message on failure.
+ * each segment's state is stepped forward from its checkpoint and kept every few
+ * levels in d_states (room for `every` fields), then the adjoint steps
+ * lambda_n = lambda_{n+1} + L(C .* lambda_{n+1}), dJ/dC += lambda_{n+1} .* L u_n
+ * run backward through it, those few levels per launch.  d_lamwork is a scratch
+ * field.  `err` receives a message on failure.
  *
  * ps_heatvar_courant: only the courant field, d_courant = d_alpha*dt/dx/dx
  * (the values ps_heatvar_forward writes), for the swept form of the same
@@ -326,9 +330,8 @@ const char *ps_batch_last_error(const ps_batch *b);
  * swept adjoint: from d_u0 (the segment's checkpoint) runs `length` steps and
  * stores the Laplacian of every old level k = 0 .. length-1 at
  * d_lap[k][nx][ny] (the field 1 that PS_EQ_HEATVAR_ADJ(MU) solvers read);
- * d_work holds two fields of scratch.  Two steps per launch, the fused
- * forward kernels' arithmetic, so the Laplacians equal those the
- * PS_EQ_HEATVAR solver stores.
+ * d_work holds two fields of scratch.  The forward kernels' arithmetic, so the
+ * Laplacians equal those the PS_EQ_HEATVAR solver stores.
  */
 int ps_heatvar_courant(const double *d_alpha, double *d_courant, int nx, int ny, double dt,
                        double dx, void *stream, char *err, size_t errlen);

@@ -30,27 +30,25 @@ def _call(fn, *args):
 
 
 class SweptHeatVar:
-    """The same solve through the swept decomposition (the engine's prism,
-    bridge and octahedron phases; Engine equations "heatvar",
-    "heatvar_adjoint_mu" and "heatvar_adjoint", csrc/equations.cuh):
+    """The same solve through the swept engine (Engine equations "heatvar",
+    "heatvar_adjoint_mu" and "heatvar_adjoint": overlapped tiles of several
+    levels per launch, csrc/heatvar_block.cuh; the prism, bridge and octahedron
+    phases where their fields are not 16-byte aligned):
 
     * forward: u0 -> u_T with a courant number per cell, the state copied out
       every `every` steps (the checkpoints);
     * backward: for the segments from the last to the first, the segment's
       levels are recomputed from its checkpoint, storing each old level's
-      Laplacian L(u_n) (ps_heatvar_recompute: the fused two-level forward
-      kernels, faster than the swept forward where the fields fit in L2, and
-      the same values); then an adjoint engine runs the segment backward
-      through the swept decomposition.
+      Laplacian L(u_n) (ps_heatvar_recompute: the forward kernels' values);
+      then an adjoint engine runs the segment backward.
 
     form="mu" (default): the adjoint in mu = C .* lambda,
-    mu_n = mu_{n+1} + C .* L(mu_{n+1}), the forward step itself, so it runs in
-    the forward's register-resident streams; the sum of mu_{n+1} .* L(u_n)
+    mu_n = mu_{n+1} + C .* L(mu_{n+1}), the forward step itself; the sum of mu_{n+1} .* L(u_n)
     accumulates in place, and lambda_0 = mu_0 ./ C, dJ/dC = sum ./ C at the
     end.  Same gradients as the standard kernels up to rounding (the products
     C .* lambda are formed in another place).
     form="lambda": lambda_n = lambda_{n+1} + L(C .* lambda_{n+1}),
-    dJ/dC += lambda_{n+1} .* L(u_n) in the generic swept kernels; every cell
+    dJ/dC += lambda_{n+1} .* L(u_n) as two variables; every cell
     sees the standard kernels' operations in the same order, so lambda_0 and
     dJ/dalpha equal theirs bitwise.
 
@@ -136,9 +134,7 @@ class SweptHeatVar:
                 length = min(n0 + every, nsteps) - n0
                 if length <= 0:
                     continue
-                # L(u_{n0}) .. L(u_{n0+length-1}) from the checkpoint (the
-                # fused forward kernels: at sizes whose fields stay in L2 they
-                # outrun the swept forward, and the values are the same)
+                # L(u_{n0}) .. L(u_{n0+length-1}) from the checkpoint
                 _call(_lib.lib().ps_heatvar_recompute, _p(courant), _p(ck[sidx]), _p(self.lap),
                       length, nx, ny, _p(self.work))
                 a.set_global("LEN", length)
@@ -248,10 +244,10 @@ class HeatVarSolve(torch.autograd.Function):
 
 
 def heat_solve(u0, alpha, nsteps, dt, dx, every=64, swept=False):
-    """swept=False: the fused standard kernels (two levels per launch);
-    swept=True or "mu": the swept decomposition with the adjoint in
-    mu = C .* lambda (SweptHeatVar, register-resident streams); swept="lambda":
-    the swept decomposition with the adjoint in lambda, bitwise equal to the
+    """swept=False: forward tiles of several levels per launch and backward ones
+    that recompute their Laplacians on chip; swept=True or "mu": the swept
+    engine with the adjoint in mu = C .* lambda (SweptHeatVar); swept="lambda":
+    the swept engine with the adjoint in lambda, bitwise equal to the
     standard kernels.  The forward values are bitwise equal in all three."""
     if swept not in (False, True, "mu", "lambda"):
         raise ValueError(f"swept={swept!r}: False, True, 'mu' or 'lambda'")

@@ -2,9 +2,9 @@
 
 For a given equation and grid shape it times candidate tilings -- blocksize
 (8, 16, 32, 64: rows per band, which sets the maximum levels per half-cycle), levels per
-half-cycle h, and column segments per band (how many units, i.e. warps or
-CTAs, share the GPU) -- on the real shape with a short run, and keeps the
-fastest.  Every tiling computes bit-identical results (the swept decomposition
+half-cycle h, which also bounds the levels an overlapped block runs per launch,
+and column segments per band (units of the prisms) -- on the real shape with a
+short run, and keeps the fastest.  Every tiling computes bit-identical results (the swept decomposition
 is exact for any tiling), so the choice only affects speed.  Results are cached
 per (equation, shape, its, GPU name) in a JSON file (``$PYSWEEP_B200_CACHE``
 or ``~/.cache/pysweep_b200/autotune.json``).
@@ -70,9 +70,9 @@ def _globals(equation, n):
 
 
 def register_streams(equation, ny, its, bs):
-    """Whether the library runs this shape on its register-resident heat
-    streams (any segment count up to ny/32); the generic streams need ny to
-    be a multiple of the segment count."""
+    """Whether the library runs this shape in blocks of their own size and
+    takes any segment count up to ny/32; elsewhere ny has to be a multiple of
+    the segment count."""
     return equation == "heat" and its == 1 and bs in (16, 32) and ny % 32 == 0
 
 

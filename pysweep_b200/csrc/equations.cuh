@@ -348,8 +348,8 @@ struct HeatVarAdj {
 // reads L(u_n), n = segment end - gts, at f[1][(i[3]-gts)*fs + row*ny + col]
 // and adds mu_{n+1} * L(u_n) to f[2][row*ny + col] in place (one fused
 // multiply-add per cell and level, in level order in every decomposition).
-// The register-resident streams (heat_fast.cuh, per-cell courant) do the
-// same arithmetic.  i[1] = nx, i[2] = ny.
+// The overlapped tiles (heatvar_block.cuh) do the same arithmetic.  i[1] = nx,
+// i[2] = ny.
 struct HeatVarAdjMu {
     static constexpr int OPS = 1;
     static constexpr int ID = EQ_HEATVAR_ADJMU;

@@ -29,7 +29,7 @@
 //       strips (a strip's 2 T rows of run-in weigh more than the tile's), for
 //       the levels left over by T = 8 and for levels kept as frames.
 //
-// Global traffic per cell and 8 levels: one read (1.14x) and one write, 2.1
+// Global traffic per cell and 8 levels: one read (1.14x) and one write, 2.0
 // bytes per cell and level.
 #pragma once
 #include <algorithm>

@@ -394,14 +394,13 @@ int ensure_swept_buffers(ps_solver* s)
 }
 
 // Levels per half-cycle until configured: MPSS, except heat with forward
-// Euler at bs 32, whose register streams run fastest at 12 of the 15
-// possible levels (measured on B200 at 4096² and 8192²: 3.8% and 6.9% over
-// 15; the prism's last levels hold 2-6 rows and are pure latency).  Results
+// Euler at bs 32.  The prisms, the row slabs' halo exchange and the adjoint's
+// checkpoint segments count in them; overlapped blocks take as many levels per
+// launch as suit the grid.  12 of 15 is what heat's callers have always been
+// told (ps_get_tiling): saved tilings and segment lengths stay valid.  Results
 // do not depend on the choice.
 int default_levels(int eq, int its, int bs, int mpss)
 {
-    // heat with forward Euler and the per-cell-courant variants share the
-    // register streams, measured fastest at 12 levels for blocksize 32
     if ((eq == PS_EQ_HEAT || eq == PS_EQ_HEATVAR || eq == PS_EQ_HEATVAR_ADJMU) && its == 1 && bs == 32)
         return std::min(mpss, 12);
     return mpss;
@@ -687,7 +686,7 @@ int run_levels(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t 
 // Euler level by level (euler_march.cuh), for either decomposition: its levels
 // are bound by arithmetic, not by memory, so a cell evaluated twice costs more
 // than a level kept on chip saves (prisms of blocksize 16 at 4096²: 6.3 G cell
-// stages/s, at 1120² 5.1; level by level 18.7 and 16.0).
+// stages/s, at 1120² 5.1; level by level 21.4 and 18.7).
 int run_march(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t frame_cap,
               int frame_every, int kind)
 {
@@ -1527,8 +1526,8 @@ int ps_configure(ps_solver* s, int h, int nseg, int chunk, int threads)
         s->chunk = chunk;
     }
     if (threads) {
-        // 128: register-resident heat streams where they apply (default);
-        // 256: always the generic shared-memory streams
+        // 128: overlapped blocks and level-by-level kernels where they apply
+        // (default); 256: always the shared-memory prisms
         if (threads != 256 && threads != 128)
             return fail(s, PS_ERR_UNSUPPORTED, "threads must be 128 or 256");
         s->threads = threads;
@@ -2194,12 +2193,10 @@ int ps_batch_create(ps_batch** out, int device, int equation, int count, const i
         else if (!b->fast && 32 < 2 * ops * (b->H + 1))
             rc = bfail(b, PS_ERR_UNSUPPORTED, "blocksize %d too large for the batched streams", blocksize);
         I.nb = I.nx / blocksize;
-        // register streams: segments of about 512 columns (measured: 256 heat
-        // instances of 128-2048², 1000 steps, 0.998 s at 256 columns, 0.845 s
-        // at 512; narrower segments multiply the seam work per cell).  The
-        // generic streams: segments of about 256 columns that divide ny and
-        // hold a chunk, so that the units of large and small instances take
-        // similar times (a phase waits for its slowest unit)
+        // heat in blocks needs no segments (the count is only reported); the
+        // prisms: segments of about 256 columns that divide ny and hold a
+        // chunk, so that the units of large and small instances take similar
+        // times (a phase waits for its slowest unit)
         if (b->fast) {
             I.nseg = std::max(1, I.ny / 512);
         } else {

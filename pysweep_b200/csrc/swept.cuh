@@ -79,9 +79,8 @@ __device__ __forceinline__ int wrap(int v, int n)
 }
 
 // Column of the x-face buffers that holds grid column g at level m: faces are
-// stored shifted by m columns, so that the register streams, whose chunks
-// slide one column left per level, write and read every level's faces at the
-// chunk's level-0 columns (16-byte aligned pairs).  All kernels use it.
+// stored shifted by m columns: the streams' chunks slide one column left per
+// level, so every level's faces lie at the chunk's level-0 columns.
 __device__ __forceinline__ int xface_col(int g, int m, int ny)
 {
     const int c = g + m;
