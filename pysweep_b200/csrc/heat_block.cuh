@@ -433,10 +433,16 @@ struct TileShape {
     int C, R, nw, maxw;
 };
 
-constexpr TileShape kTilesFE[] = {{4, 6, 16, 16}, {4, 6, 12, 16}, {4, 6, 8, 16}, {2, 8, 12, 20},
-                                  {2, 8, 8, 20},  {2, 8, 6, 20},  {2, 4, 12, 24}, {2, 4, 8, 24},
-                                  {2, 4, 6, 24},  {2, 4, 4, 24}};
-constexpr TileShape kTilesRK2[] = {{4, 4, 16, 16}, {4, 4, 12, 16}, {4, 4, 8, 16},
+// (eight and ten rows of four columns: grids whose tiles then fit the SMs in
+// fewer rounds, 1000 x 1400 1.73 -> 1.51 us per level, 1280² 1.95 -> 1.75)
+constexpr TileShape kTilesFE[] = {{4, 6, 16, 16}, {4, 6, 12, 16}, {4, 6, 8, 16},  {4, 8, 16, 16},
+                                  {4, 10, 12, 12}, {2, 8, 12, 20}, {2, 8, 8, 20}, {2, 8, 6, 20},
+                                  {2, 4, 12, 24}, {2, 4, 8, 24},  {2, 4, 6, 24},  {2, 4, 4, 24}};
+// Two stages keep two fields in registers.  us per level with four rows of four
+// columns and 16 warps, before / with these: 512² 0.95 / 0.60, 1120² 1.80 /
+// 1.51, 1000 x 1400 1.95 / 1.84, 1536² 3.0 / 2.78.
+constexpr TileShape kTilesRK2[] = {{4, 8, 12, 12}, {4, 6, 12, 12}, {4, 4, 16, 16},
+                                   {2, 8, 16, 16}, {2, 8, 12, 16}, {2, 8, 8, 16},
                                    {2, 4, 12, 24}, {2, 4, 8, 24},  {2, 4, 6, 24}};
 
 // How a run of levels is cut into launches: streams of kStreamT levels (and
@@ -476,9 +482,17 @@ struct BlockGrids {
 // tile, latency of a level.  two: a level of tiles of two columns and eight rows,
 // whose warps exchange more per cell (1280²: 2.17 us per level where six rows of
 // four columns take 1.96; without it they were planned at 1.95 and 1.98).
+// four: one of tiles of four rows.  stream: a launch of the streams.
 struct TileCost {
-    double level = 1.0, bytes = 1.0, latency = 1.0, two = 1.1;
+    double level = 1.0, bytes = 1.0, latency = 1.0, two = 1.1, four = 1.0, stream = 1.0;
 };
+// Two stages: fitted to launches of 160² to 2048² (the plan within 1% of the best
+// tile there).
+constexpr TileCost kCostRK2{1.0, 1.17, 1.0, 1.1, 1.15, 1.0};
+// float32 fields: two conversions per cell and level, which the streams' warps
+// hide better than a tile's (2048², float64 / float32, us per 8 levels: streams
+// 32.2 / 36.6, tiles 36.4 / 46.7).
+constexpr TileCost kCostF32{1.0, 1.0, 1.0, 1.1, 1.0, 0.91};
 
 // Estimated microseconds of one launch of T levels in tiles of shape t, or 0
 // where no cell of the tile stays exact.  Fitted to launches of 160² to 8192²
@@ -494,7 +508,9 @@ inline double tile_us(const TileShape& t, int T, const BlockGrids& g, int sms,
     const double n = (double)((g.blocks(vw, vh) + sms - 1) / sms);  // tiles of the busiest SM
     const int occ = t.maxw / t.nw;
     const double k = std::min(n, (double)occ), rounds = std::max(1.0, n / occ);
-    const double level = 4.0 * t.nw * t.R * t.C / 1965.0 * 1.04 * c.level * (t.C == 2 && t.R == 8 ? c.two : 1.0);
+    const double level = 4.0 * t.nw * t.R * t.C / 1965.0 * 1.04 * c.level * (t.C == 2 && t.R == 8 ? c.two : 1.0) *
+                         (t.R == 4 ? c.four : 1.0) *
+                         (t.maxw <= 12 ? 0.95 : 1.0);  // (registers to overlap rows)
     const double kb = k * t.nw * t.R * t.C * 32 * 8 / 1024.0 * 0.03 * c.bytes;
     const double lat = (k * t.nw <= 12 ? 0.08 : 0.03) * c.latency;
     return 1.0 + n * T * level + (occ == 1 ? rounds : 1.0) * kb + (n - k) * 0.4 + lat * T * rounds;
@@ -546,22 +562,22 @@ inline BlockPlan plan_tiles(const TileShape (&shapes)[NSHAPE], const BlockGrids&
     return best;
 }
 
-// The cheapest way to run nlevels levels.  Streams win from about 1700² up
-// (us per level, stream / best tile: 1120² 2.08 / 1.33, 2048² 4.02 / 4.31,
+// The cheapest way to run nlevels levels.  Streams win from about 2000² up
+// (us per level, stream / best tile: 1120² 2.08 / 1.33, 2048² 4.02 / 4.05,
 // 4096² 11.6 / 15.7, 8192² 42.4 / 60.0); below, the tile whose count fits the
 // SMs best.
 template <int NSHAPE>
 inline BlockPlan plan_block(const TileShape (&shapes)[NSHAPE], const BlockGrids& g, int nlevels,
-                            int step, int maxT, int sms)
+                            int step, int maxT, int sms, const TileCost& cost = TileCost{})
 {
-    BlockPlan best = plan_tiles(shapes, g, nlevels, step, maxT, sms);
+    BlockPlan best = plan_tiles(shapes, g, nlevels, step, maxT, sms, cost);
     if (nlevels >= kStreamT && maxT >= kStreamT) {
         const int rows = stream_rows(g, sms);
         // (strips of very wide grids, or of many, may fill more than one wave)
         const double waves = std::max(1.0, (double)g.blocks(kStreamW, rows) / (8.0 * sms));
-        double us = nlevels / kStreamT * (10.2 + 0.645 * rows) * waves, tail = 0.0;
+        double us = nlevels / kStreamT * (10.2 + 0.645 * rows) * waves * cost.stream, tail = 0.0;
         const int rest = (nlevels % kStreamT + step - 1) / step * step;
-        if (rest) best_tile(shapes, rest, g, sms, &tail);
+        if (rest) best_tile(shapes, rest, g, sms, &tail, cost);
         if (us + tail < best.us) best = BlockPlan{true, kStreamT, us + tail};
     }
     return best;
@@ -595,10 +611,15 @@ inline void launch_block_tile(const TileShape& t, BlockArgs a, int T, cudaStream
     a.ncs = (a.ny + a.vw - 1) / a.vw;
     a.units = a.ncs * ((a.nx + a.vh - 1) / a.vh);
     if constexpr (RK2) {
-        if (t.C == 4) launch_tile<S, RK2, 4, 4, 16>(a, t.nw, st);
+        if (t.C == 4 && t.R == 8) launch_tile<S, RK2, 4, 8, 12>(a, t.nw, st);
+        else if (t.R == 6) launch_tile<S, RK2, 4, 6, 12>(a, t.nw, st);
+        else if (t.C == 4) launch_tile<S, RK2, 4, 4, 16>(a, t.nw, st);
+        else if (t.R == 8) launch_tile<S, RK2, 2, 8, 16>(a, t.nw, st);
         else launch_tile<S, RK2, 2, 4, 24>(a, t.nw, st);
     } else {
-        if (t.C == 4) launch_tile<S, RK2, 4, 6, 16>(a, t.nw, st);
+        if (t.R == 10) launch_tile<S, RK2, 4, 10, 12>(a, t.nw, st);
+        else if (t.C == 4 && t.R == 8) launch_tile<S, RK2, 4, 8, 16>(a, t.nw, st);
+        else if (t.C == 4) launch_tile<S, RK2, 4, 6, 16>(a, t.nw, st);
         else if (t.R == 8) launch_tile<S, RK2, 2, 8, 20>(a, t.nw, st);
         else launch_tile<S, RK2, 2, 4, 24>(a, t.nw, st);
     }

@@ -528,8 +528,9 @@ int run_block(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
     a.cr = prm.d[0];
     if (done < last) {
         const int n = (int)std::min<int64_t>(last - done, 1 << 20);
-        if constexpr (RK2) plan = plan_block(kTilesRK2, grids, n, step, maxT, sms);
-        else plan = plan_block(kTilesFE, grids, n, step, maxT, sms);
+        const TileCost cost = RK2 ? kCostRK2 : (sizeof(S) == 4 ? kCostF32 : TileCost{});
+        if constexpr (RK2) plan = plan_block(kTilesRK2, grids, n, step, maxT, sms, cost);
+        else plan = plan_block(kTilesFE, grids, n, step, maxT, sms, cost);
     }
     // frames are stored by the block that computes their level where 4-wide
     // stores may reach them; else the block ends at the level and it is copied
@@ -557,7 +558,7 @@ int run_block(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
                  if (tile) {
                      double us;
                      if constexpr (RK2)
-                         launch_block_tile<S, RK2>(best_tile(kTilesRK2, T, grids, sms, &us), a, T, s->stream);
+                         launch_block_tile<S, RK2>(best_tile(kTilesRK2, T, grids, sms, &us, kCostRK2), a, T, s->stream);
                      else
                          launch_block_tile<S, RK2>(best_tile(kTilesFE, T, grids, sms, &us), a, T, s->stream);
                  } else {
@@ -2044,6 +2045,8 @@ int batch_block_enqueue(ps_batch* b, const std::vector<BlockStep>& steps)
         if (s.stream)
             launch_after(heat_block_stream_batch<double>, t.n, 32, 0, b->stream, (const BlockInst*)b->d_binst,
                          (const int2*)t.d, par, t.vh);
+        else if (s.tile.R == 10) launch_tile_batch<4, 10, 12>(b, s, t, par);
+        else if (s.tile.C == 4 && s.tile.R == 8) launch_tile_batch<4, 8, 16>(b, s, t, par);
         else if (s.tile.C == 4) launch_tile_batch<4, 6, 16>(b, s, t, par);
         else if (s.tile.R == 8) launch_tile_batch<2, 8, 20>(b, s, t, par);
         else launch_tile_batch<2, 4, 24>(b, s, t, par);

@@ -102,6 +102,25 @@ def test_streams(nx, ny, bs, its, nl):
     assert all(np.array_equal(a, b) for a, b in zip(got, ref))
 
 
+@pytest.mark.parametrize("nx,ny,bs,its,nl", [
+    (1000, 1400, 8, 1, 23), (1280, 1280, 32, 1, 16), (1664, 1664, 32, 1, 25),
+    (512, 512, 16, 2, 20), (702, 702, 6, 2, 17), (1000, 1400, 8, 2, 24), (1120, 1120, 16, 2, 9)])
+def test_tiles_of_many_rows(nx, ny, bs, its, nl):
+    """Grids whose plan takes the tiles of eight and ten rows per warp, alone and
+    as a batch of one."""
+    from pysweep_b200 import Batch, plugin_constants
+    ic, g = _ic(nx, ny), _globals(nx, its == 1)
+    got, _ = _solve(ic, g, its, bs, nl)
+    ref, _ = _solve(ic, g, its, bs, nl, mode="standard", threads=256)
+    assert all(np.array_equal(a, b) for a, b in zip(got, ref))
+    if its == 1 and nx % 32 == 0:
+        with Batch("heat", [(nx, ny)], blocksize=bs) as b:
+            b.set_constants(0, plugin_constants("heat", g))
+            b.set_state(0, ic)
+            b.run(nl)
+            assert np.array_equal(b.get_state(0), ref[0])
+
+
 @pytest.mark.parametrize("h", [1, 2, 5])
 def test_configured_levels_bound_a_launch(h):
     nx, ny, nl = 96, 160, 11
