@@ -797,13 +797,14 @@ int run_heat_standard(ps_solver* s, int64_t nlevels, int gts0, double* frames, i
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
     const double cr = make_params(s).d[0];
     const int rows = standard_rows(s->nx, s->ny, sms);
-    const int units = (s->ny + 63) / 64 * ((s->nx + rows - 1) / rows);
+    const int below = standard_below(RK2, s->nx, s->ny);
+    const int grid = standard_grid(s->nx, s->ny, rows, below);
     return run_levels(s, nlevels, gts0, frames, frame_cap, frame_every, 4,
                       [&](const double* cur, const double* prev, double* out, double* fr, int gts) {
                           launch_after(rows == 4 ? heat_standard<RK2, 4, T> : heat_standard<RK2, 8, T>,
-                                       (units + kStdWarps - 1) / kStdWarps, 32 * kStdWarps, 0,
+                                       grid, 32 * kStdWarps, 0,
                                        s->stream, (const T*)cur, (const T*)prev, (T*)out, (T*)fr,
-                                       s->nx, s->ny, gts, cr);
+                                       s->nx, s->ny, gts, cr, below);
                       });
 }
 

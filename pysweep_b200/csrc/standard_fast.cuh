@@ -9,8 +9,8 @@
 // Bound by HBM where the fields exceed L2 (16 bytes per cell: 428 G cells/s at
 // 8192², 106% of the measured copy's rate, the halo rows coming from L2), below
 // by the launch and one round trip.  us per level, against rows streamed one by
-// one down 32-row strips: 2048² 14.4 -> 7.4, 4096² 49 -> 41, 8192² 182 -> 157;
-// against one thread per cell (1120 columns are no multiple of 64): 7.4 -> 3.5.
+// one down 32-row strips: 2048² 14.4 -> 7.2, 4096² 49 -> 41, 8192² 182 -> 157;
+// against one thread per cell (1120 columns are no multiple of 64): 7.4 -> 3.3.
 // T is the storage type (double, or float with every level evaluated in
 // double and rounded to float, as the reference's float32 runs do).
 #pragma once
@@ -21,10 +21,23 @@ namespace psb {
 constexpr int kStdWarps = 4;
 
 // Rows per warp: eight; four where eight leave the SMs fewer than 28 warps each
-// (1120²: 3.5 against 3.8 us; 2048²: 7.75 against 7.4).
+// (1120²: 3.5 against 3.8 us; 2048²: 7.75 against 7.4; before the warps were stacked).
 inline int standard_rows(int nx, int ny, int sms)
 {
     return (long long)((ny + 63) / 64) * ((nx + 7) / 8) < 28LL * sms ? 4 : 8;
+}
+
+// Whether a CTA's warps lie below one another, so that the rows they share come
+// from L1, or side by side (us, side by side / below: 1152² 3.7 / 3.5, float32 4.0 /
+// 3.3, 2048² 7.5 / 7.3; where a field is far larger than L2 8192² 156 / 159; where a
+// full stage reads a second field 2048² 10.7 / 11.9).
+inline bool standard_below(bool rk2, int nx, int ny) { return !rk2 && (long long)nx * ny <= 1 << 24; }
+
+// CTAs of a level in rows of `rows` per warp.
+inline int standard_grid(int nx, int ny, int rows, bool below)
+{
+    const int ncs = (ny + 63) / 64, nr = (nx + rows - 1) / rows;
+    return below ? ncs * ((nr + kStdWarps - 1) / kStdWarps) : (ncs * nr + kStdWarps - 1) / kStdWarps;
 }
 
 template <bool RK2, int RB, class T>
@@ -32,17 +45,20 @@ __global__ void __launch_bounds__(32 * kStdWarps) heat_standard(const T* __restr
                                                                 const T* __restrict__ prev,
                                                                 T* __restrict__ out,
                                                                 T* __restrict__ frame, int nx,
-                                                                int ny, int gts, double cr)
+                                                                int ny, int gts, double cr, int below)
 {
     using P = typename Pair2<T>::type;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ncs = (ny + 63) / 64;
-    const int unit = blockIdx.x * kStdWarps + warp;
-    const int x0 = unit / ncs * RB;
+    const int unit = below ? blockIdx.x : blockIdx.x * kStdWarps + warp, row = unit / ncs;
+    const int x0 = below ? (row * kStdWarps + warp) * RB : row * RB;
     if (x0 >= nx) return;  // whole warp
-    const int c0 = unit % ncs * 64 + 2 * lane;  // (the last strip may reach past the row: it wraps)
-    const int g = wrap(c0, ny);
-    const int hcol = lane == 0 ? wrap(c0 - 1, ny) : wrap(c0 + 2, ny);
+    const int c0 = (unit - row * ncs) * 64 + 2 * lane;
+    // (the last strip may reach past the row: it wraps; what lies further than
+    // one row on, nobody reads)
+    auto in_row = [&](int c) { return c < ny ? c : (c < 2 * ny ? c - ny : 0); };
+    const int g = in_row(c0);
+    const int hcol = lane == 0 ? (c0 == 0 ? ny - 1 : in_row(c0 - 1)) : in_row(c0 + 2);
     const bool edge = lane == 0 || lane == 31;
     const bool full = (gts % 2 == 0);
     grid_wait();
