@@ -101,9 +101,8 @@ struct HookFrames {
 };
 
 extern "C" __global__ void __launch_bounds__(psb::kBlkNT)
-    psh_block(const double* __restrict__ newest, const double* __restrict__ older,
-              double* __restrict__ out, double* __restrict__ out1, HookFrames frames, int any_frame,
-              int nx, int ny, int T, int rows1, int gts)
+    psh_block(const double* newest, const double* older, double* out, double* out1,
+              HookFrames frames, int any_frame, int nx, int ny, int T, int rows1, int gts)
 {
     using namespace psb;
     constexpr int OPS = PSH_OPS, NV = PSH_NV, CC = kBlkCols;

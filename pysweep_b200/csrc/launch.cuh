@@ -26,7 +26,11 @@ void allow_big_smem(K kernel)
 }
 
 // A kernel that may begin while the one before it in the stream ends (it waits
-// for it itself: grid_wait).
+// for it itself: grid_wait).  Its fields come in through plain pointers, never
+// const __restrict__ ones: that promises that nobody writes the data while the
+// kernel lives, which the kernel before it still does, and lets the compiler
+// load it through the non-coherent path or above the wait (whose memory clobber
+// orders no load of data promised not to change).
 template <class... P, class... A>
 void launch_after(void (*k)(P...), int grid, int nt, size_t smem, cudaStream_t st, A... args)
 {

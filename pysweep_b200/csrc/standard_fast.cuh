@@ -41,11 +41,9 @@ inline int standard_grid(int nx, int ny, int rows, bool below)
 }
 
 template <bool RK2, int RB, class T>
-__global__ void __launch_bounds__(32 * kStdWarps) heat_standard(const T* __restrict__ cur,
-                                                                const T* __restrict__ prev,
-                                                                T* __restrict__ out,
-                                                                T* __restrict__ frame, int nx,
-                                                                int ny, int gts, double cr, int below)
+__global__ void __launch_bounds__(32 * kStdWarps) heat_standard(const T* cur, const T* prev,
+                                                                T* out, T* frame, int nx, int ny,
+                                                                int gts, double cr, int below)
 {
     using P = typename Pair2<T>::type;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
