@@ -1974,7 +1974,10 @@ int batch_table(ps_batch* b, int vw, int vh, int* index)
     }
     int2* d = nullptr;
     PSB_CUDA(b, cudaMalloc(&d, u.size() * sizeof(int2)));
-    cudaError_t e = cudaMemcpy(d, u.data(), u.size() * sizeof(int2), cudaMemcpyHostToDevice);
+    // (on the batch's own stream: it does not wait for the legacy one, and a copy
+    // from pageable memory may return before it lands)
+    cudaError_t e = cudaMemcpyAsync(d, u.data(), u.size() * sizeof(int2), cudaMemcpyHostToDevice, b->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) {
         cudaFree(d);
         return bfail(b, PS_ERR_CUDA, "block table: %s", cudaGetErrorString(e));
@@ -2249,7 +2252,9 @@ int ps_batch_create(ps_batch** out, int device, int equation, int count, const i
             e = cudaMalloc(&b->d_minst, b->inst.size() * sizeof(MarchInst));
         if (e == cudaSuccess) e = cudaMalloc(&b->d_units, units.size() * sizeof(int2));
         if (e == cudaSuccess)
-            e = cudaMemcpy(b->d_units, units.data(), units.size() * sizeof(int2), cudaMemcpyHostToDevice);
+            e = cudaMemcpyAsync(b->d_units, units.data(), units.size() * sizeof(int2),
+                                cudaMemcpyHostToDevice, b->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
         if (e != cudaSuccess) rc = bfail(b, PS_ERR_NOMEM, "batch tables: %s", cudaGetErrorString(e));
     }
     // the kernels of the chosen chunk width (prep opts them into large shared memory)

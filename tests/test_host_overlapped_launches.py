@@ -1,7 +1,8 @@
 """Rules of kernels that begin while the one before them in the stream ends
-(programmatic dependent launches), checked in their source: no GPU needed.
+(programmatic dependent launches), and of the copies they read, checked in the
+source: no GPU needed.
 
-Such a kernel's fields are written by the kernel before it while it already
+An overlapped kernel's fields are written by the kernel before it while it already
 lives, so it must not take them through __restrict__ pointers: the compiler may
 then load them through the non-coherent path, or above the wait.  Tables of
 descriptors and units are written by copies that end before the launch begins."""
@@ -48,3 +49,12 @@ def test_overlapped_kernels_promise_nothing_about_their_fields():
                     assert kind in TABLES, f"{f}: {name}: {p.strip()}"
     assert {"heat_standard", "heat_block_stream", "heat_block_tile", "heat_block_tile_batch",
             "heatvar_tile", "heatvar_back", "euler_march", "euler_march_batch", "psh_block"} <= set(seen)
+
+
+def test_device_data_is_copied_on_the_stream_that_reads_it():
+    """Solvers and batches run on non-blocking streams, which the legacy stream's
+    copies do not wait for and are not waited for by; one from pageable memory may
+    return before it lands."""
+    for f in sorted(os.listdir(CSRC)):
+        text = re.sub(r"//.*", "", open(os.path.join(CSRC, f)).read())
+        assert not re.search(r"\bcuda(Memcpy|Memset|Memcpy2D|MemcpyToSymbol)\s*\(", text), f
