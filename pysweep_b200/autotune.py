@@ -4,13 +4,15 @@ For a given equation and grid shape it times candidate tilings -- blocksize
 (8, 16, 32, 64: rows per band, which sets the maximum levels per half-cycle), levels per
 half-cycle h, which also bounds the levels an overlapped block runs per launch,
 and column segments per band (units of the prisms) -- on the real shape with a
-short run, and keeps the fastest.  Every tiling computes bit-identical results (the swept decomposition
-is exact for any tiling), so the choice only affects speed.  Results are cached
+short run, and keeps the fastest.  The library's own tiling of every blocksize
+(h and nseg 0: nothing configured, blocks as deep as suits the grid) comes first.
+Every tiling computes bit-identical results (the swept decomposition is exact for
+any tiling), so the choice only affects speed.  Results are cached
 per (equation, shape, its, GPU name) in a JSON file (``$PYSWEEP_B200_CACHE``
 or ``~/.cache/pysweep_b200/autotune.json``).
 
     from pysweep_b200.autotune import tune
-    best = tune("heat", 8192, 8192)      # {"blocksize": 32, "h": 15, "nseg": 6, ...}
+    best = tune("heat", 8192, 8192)      # {"blocksize": 32, "h": 0, "nseg": 0, ...}
     eng = Engine("heat", 8192, 8192, blocksize=best["blocksize"])
     eng.configure(h=best["h"], nseg=best["nseg"])
 """
@@ -142,7 +144,12 @@ def tune(equation, nx, ny, nv=None, its=1, ops=None, levels=None, reps=2, device
     dfield = torch.from_numpy(field).cuda(device)
     levels = levels or 60 * its
     results = []
-    for bs, h, nseg in candidates(equation, nx, ny, its, ops, blocksizes):
+    tilings = candidates(equation, nx, ny, its, ops, blocksizes)
+    # the library's own first: a configured h caps its blocks (heat, us per level
+    # unset / highest h: 1000 x 1400, blocksize 8, 1.55 / 2.21; 4096², blocksize 16,
+    # 11.6 / 16.1)
+    own = [(bs, 0, 0) for bs in dict.fromkeys(t[0] for t in tilings)]
+    for bs, h, nseg in own + tilings:
         try:
             g = _time_config(equation, nx, ny, nv, its, ops, bs, h, nseg, levels, reps, device,
                              dfield)
