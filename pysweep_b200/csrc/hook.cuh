@@ -34,37 +34,55 @@ enum HookFw { FW_VARS, FW_TIMES, FW_MPSS, FW_MOSS, FW_NV, FW_OPS, FW_ITS, FW_SX,
 constexpr const char* kHookFw[FW_COUNT] = {"VARS", "TIMES", "MPSS", "MOSS", "NV",
                                            "OPS",  "ITS",   "SX",   "SY"};
 // block tiles of the hook kernels (hook_kernels.cuh): columns of level 1, most
-// threads, most levels per launch.  Several levels run 512 threads (a step's
-// loads may not pass the store of the step before it, so warps have to cover
-// its latency; heat at 1024², us per level with 256 / 512 / 1024: 5.2, 4.6, 6.6),
-// one level 256 (8.5, 10.5, 15.9).
+// threads, most levels per launch.
 constexpr int kHookBlkW = 64, kHookBlkNT = 512, kHookBlkMaxT = 8;
 
-// Rows of level 1 and levels of a block, or rows 0 where no tile fits.  Slots
-// of levels -1 .. T; the deepest block whose last level keeps two thirds of the
-// first one's cells and whose tile leaves room for two CTAs per SM; one level
-// (any room) where a second does not fit.
+// Rows of level 1 and levels of a block, threads of a launch of one level (of
+// several: kHookBlkNT), or rows 0 where no tile fits.
+// Slots of levels -1 .. T; the deepest block whose last level keeps two thirds of
+// the first one's cells and whose tile leaves room for two CTAs per SM; one level
+// where a second does not fit.  Several levels run 512 threads (a step's loads may
+// not pass the store of the step before it, so warps have to cover its latency;
+// heat at 1024², us per level with 256 / 512 / 1024: 5.2, 4.6, 6.6).
+//
+// One level: as many rows as leave enough warps on an SM, a warp to a row.  A
+// stencil of nv variables and reach ops, us per level with 32 rows and 256 threads
+// / 16 and 256 / 8 and 256 / 16 and 512 (-: too large):
+//     512²  nv 1 ops 1  7.8 / 6.3 / 5.9 / 5.9   nv 3 ops 2    - /  13 /  15 /  12
+//     2048² nv 1 ops 1   42 /  44 /  53 /  60   nv 3 ops 2    - / 167 / 143 / 136
+//           nv 2 ops 1  105 /  76 /  78 /  86   nv 4 ops 1    - / 209 / 146 / 177
+//           nv 4 ops 2    - /   - / 240 / 267   nv 6 ops 2    - /   - / 569 / 373
+// so 32 rows where four CTAs fit on an SM and there are eight for each, 16 where
+// three fit; else 16 with 512 threads where two do and the halo is wide (eight rows
+// load half as much again), 8 where two do, 16 with 512 threads where one does.
 struct HookBlock {
-    int rows, T;
+    int rows, T, threads1;
 };
-inline int hook_block_threads(int T) { return T > 1 ? kHookBlkNT : kHookBlkNT / 2; }
 inline size_t hook_block_smem(int nv, int ops, int rows, int T)
 {
     return sizeof(double) * (T + 2) * nv * (rows + 2 * ops) * (kHookBlkW + 2 * ops);
 }
-inline HookBlock hook_block(int nv, int ops, int maxT)
+inline HookBlock hook_block(int nv, int ops, int maxT, long long cells, int sms)
 {
+    constexpr int few = kHookBlkNT / 2;
     for (int rows : {32, 16})
         for (int T = maxT < kHookBlkMaxT ? maxT : kHookBlkMaxT; T >= 2; --T) {
             const int ih = rows - 2 * ops * (T - 1), iw = kHookBlkW - 2 * ops * (T - 1);
             const size_t sm = hook_block_smem(nv, ops, rows, T);
             if (ih > 0 && iw > 0 && 3 * ih * iw >= 2 * rows * kHookBlkW && sm <= 113 * 1024)
-                return HookBlock{rows, T};
+                return HookBlock{rows, T, few};
         }
-    for (int rows : {32, 16, 8, 4})
-        if (hook_block_smem(nv, ops, rows, 1) <= (rows > 8 ? 113 : 227) * 1024)
-            return HookBlock{rows, 1};
-    return HookBlock{0, 0};
+    auto fit = [&](int rows) {  // CTAs on an SM: 228 KB, 1 KB for each besides its own
+        return (int)(228 * 1024 / (hook_block_smem(nv, ops, rows, 1) + 1024));
+    };
+    if (fit(32) >= 4 && cells >= 8LL * sms * 32 * kHookBlkW) return HookBlock{32, 1, few};
+    if (fit(16) >= 3) return HookBlock{16, 1, few};
+    if (fit(16) >= 2 && ops >= 2) return HookBlock{16, 1, kHookBlkNT};
+    if (fit(8) >= 2) return HookBlock{8, 1, few};
+    if (fit(16) >= 1) return HookBlock{16, 1, kHookBlkNT};
+    for (int rows : {8, 4})
+        if (fit(rows) >= 1) return HookBlock{rows, 1, few};
+    return HookBlock{0, 0, 0};
 }
 
 // A user constant, in every namespace (ps_get_global hands out a pointer to

@@ -735,7 +735,7 @@ void hook_block_launch(ps_solver* s, const HookBlock& b, int T, const double* ne
     cfg.gridDimX = (ny + iw - 1) / iw;
     cfg.gridDimY = (nx + ih - 1) / ih;
     cfg.gridDimZ = 1;
-    cfg.blockDimX = hook_block_threads(T);
+    cfg.blockDimX = T > 1 ? kHookBlkNT : b.threads1;
     cfg.blockDimY = cfg.blockDimZ = 1;
     cfg.sharedMemBytes = (unsigned)hook_block_smem(s->nv, s->ops, rows, T);
     cfg.hStream = (CUstream)s->stream;
@@ -747,6 +747,14 @@ void hook_block_launch(ps_solver* s, const HookBlock& b, int T, const double* ne
     cfg.numAttrs = 1;
     CUresult r = drv().launchKernelEx(&cfg, s->hook->block, args, nullptr);
     if (r != CUDA_SUCCESS) s->launch_err = cu_error(r);
+}
+
+// The block tiles of a solver's hook, up to maxT levels per launch.
+HookBlock solver_hook_block(const ps_solver* s, int maxT)
+{
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
+    return hook_block(s->nv, s->ops, maxT, (long long)s->nx * s->ny, sms);
 }
 
 // The framework constants of the block tiles (the same for any T).
@@ -891,7 +899,7 @@ int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
             return run_block<double, true>(s, nlevels, gts0, frames, frame_cap, frame_every, maxT);
     }
     if (s->hook && s->threads != 256) {
-        const HookBlock b = hook_block(s->nv, s->ops, s->h_set ? s->H : kHookBlkMaxT);
+        const HookBlock b = solver_hook_block(s, s->h_set ? s->H : kHookBlkMaxT);
         if (b.rows) return run_hook_block(s, b, nlevels, gts0, frames, frame_cap, frame_every);
     }
     if (s->eq == PS_EQ_EULER && s->threads != 256 && march_constants(make_params(s)))
@@ -1039,7 +1047,7 @@ int run_standard(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_
     int rc;
     HookBlock blk{};
     if (s->hook) {
-        blk = hook_block(s->nv, s->ops, 1);
+        blk = solver_hook_block(s, 1);
         if (!blk.rows) return fail(s, PS_ERR_UNSUPPORTED, "the hook's standard tile does not fit in shared memory");
         if ((rc = hook_block_frame(s, blk))) return rc;
     }
