@@ -32,8 +32,7 @@ def _call(fn, *args):
 class SweptHeatVar:
     """The same solve through the swept engine (Engine equations "heatvar",
     "heatvar_adjoint_mu" and "heatvar_adjoint": overlapped tiles of several
-    levels per launch, csrc/heatvar_block.cuh; the prism, bridge and octahedron
-    phases where their fields are not 16-byte aligned):
+    levels per launch, csrc/heatvar_block.cuh):
 
     * forward: u0 -> u_T with a courant number per cell, the state copied out
       every `every` steps (the checkpoints);

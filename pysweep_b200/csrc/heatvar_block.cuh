@@ -63,7 +63,17 @@ __device__ __forceinline__ void var_row(const double (&U)[C], const double (&M)[
     for (int j = 0; j < C; ++j) o[j] = t[j];
 }
 
-template <int ROLE, int C, int R, int MAXW>
+// two columns of a field; ODD: one by one (a field 8 bytes off a 16-byte boundary)
+template <bool ODD>
+__device__ __forceinline__ double2 ld_two(const double* p)
+{
+    return ODD ? make_double2(p[0], p[1]) : *reinterpret_cast<const double2*>(p);
+}
+
+// ODD: some field of a solver is not 16-byte aligned (2048², us per level of
+// forward, mu, lambda, aligned / odd: 5.6 / 6.1, 17.4 / 17.6, 19.0 / 19.8; the
+// shared-memory prisms 33, 49, 84).
+template <int ROLE, int C, int R, int MAXW, bool ODD>
 __global__ void __launch_bounds__(32 * MAXW, 1) heatvar_tile(const __grid_constant__ VarArgs a)
 {
     extern __shared__ __align__(16) double tile_sm[];
@@ -92,7 +102,8 @@ __global__ void __launch_bounds__(32 * MAXW, 1) heatvar_tile(const __grid_consta
 #pragma unroll
             for (int p = 0; p < NP; ++p)
                 if (ok[p]) {
-                    const double2 x = __ldcs(reinterpret_cast<const double2*>(src + 2 * p));
+                    const double2 x = ODD ? make_double2(__ldcs(src + 2 * p), __ldcs(src + 2 * p + 1))
+                                          : __ldcs(reinterpret_cast<const double2*>(src + 2 * p));
                     v[2 * p] = x.x;
                     v[2 * p + 1] = x.y;
                 }
@@ -109,8 +120,8 @@ __global__ void __launch_bounds__(32 * MAXW, 1) heatvar_tile(const __grid_consta
             const size_t o = (size_t)r * ny;
 #pragma unroll
             for (int p = 0; p < NP; ++p) {
-                const double2 v = *reinterpret_cast<const double2*>(a.in + o + gp[p]);
-                const double2 c = *reinterpret_cast<const double2*>(a.C + o + gp[p]);
+                const double2 v = ld_two<ODD>(a.in + o + gp[p]);
+                const double2 c = ld_two<ODD>(a.C + o + gp[p]);
                 u[i + 1][2 * p] = v.x;
                 u[i + 1][2 * p + 1] = v.y;
                 cr[i][2 * p] = c.x;
@@ -127,8 +138,7 @@ __global__ void __launch_bounds__(32 * MAXW, 1) heatvar_tile(const __grid_consta
 #pragma unroll
                 for (int p = 0; p < NP; ++p) {
                     double2 v = make_double2(0.0, 0.0);
-                    if (mine(i) && ok[p])
-                        v = *reinterpret_cast<const double2*>(a.g + (size_t)(r0 + i) * ny + c0 + 2 * p);
+                    if (mine(i) && ok[p]) v = ld_two<ODD>(a.g + (size_t)(r0 + i) * ny + c0 + 2 * p);
                     g[i][2 * p] = v.x;
                     g[i][2 * p + 1] = v.y;
                 }
@@ -155,7 +165,15 @@ __global__ void __launch_bounds__(32 * MAXW, 1) heatvar_tile(const __grid_consta
         }
     };
     auto store_row = [&](double* dst, int i, const double (&v)[C]) {
-        if (mine(i)) block_store<C, double>(dst + (size_t)(r0 + i) * ny, c0, clo, chi, 0, v);
+        if (!mine(i)) return;
+        double* row = dst + (size_t)(r0 + i) * ny;
+        if constexpr (ODD) {
+#pragma unroll
+            for (int j = 0; j < C; ++j)
+                if (ok[j / 2]) row[c0 + j] = v[j];
+        } else {
+            block_store<C, double>(row, c0, clo, chi, 0, v);
+        }
     };
     const int wu = w == 0 ? 0 : w - 1, wd = w == nw - 1 ? w : w + 1;
     double l[C];
@@ -304,7 +322,7 @@ BlockPlan plan_var(const BlockGrids& g, int nlevels, int sms)
 }
 
 // One launch of T levels; a: pointers, nx, ny.
-template <int ROLE>
+template <int ROLE, bool ODD = false>
 void launch_var(VarArgs a, int T, int sms, cudaStream_t st)
 {
     constexpr bool ADJ = ROLE >= VAR_LAMBDA;
@@ -321,9 +339,9 @@ void launch_var(VarArgs a, int T, int sms, cudaStream_t st)
     const int units = a.ncs * ((a.nx + a.vh - 1) / a.vh);
     const size_t smem = tile_smem<2>(t.nw);
     if (t.R == 4)
-        launch_after(heatvar_tile<ROLE, 2, 4, ADJ ? 20 : 24>, units, 32 * t.nw, smem, st, a);
+        launch_after(heatvar_tile<ROLE, 2, 4, ADJ ? 20 : 24, ODD>, units, 32 * t.nw, smem, st, a);
     else
-        launch_after(heatvar_tile<ROLE, 2, ADJ ? 6 : 8, 16>, units, 32 * t.nw, smem, st, a);
+        launch_after(heatvar_tile<ROLE, 2, ADJ ? 6 : 8, 16, ODD>, units, 32 * t.nw, smem, st, a);
 }
 
 // --------------------------------------------------------------- backward --

@@ -576,12 +576,12 @@ int run_block(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
     return PS_OK;
 }
 
-// The fields of a per-cell-courant solver can be copied 16 bytes at a time.
-bool var_aligned(const ps_solver* s)
+// Some field of a per-cell-courant solver lies off a 16-byte boundary.
+bool var_odd(const ps_solver* s)
 {
     for (const double* f : s->field)
-        if (reinterpret_cast<uintptr_t>(f) % 16) return false;
-    return s->ny % 2 == 0;
+        if (reinterpret_cast<uintptr_t>(f) % 16) return true;
+    return false;
 }
 
 // The per-cell-courant equations in overlapped tiles (heatvar_block.cuh).
@@ -605,6 +605,7 @@ int run_var(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t fra
     a.nx = s->nx;
     a.ny = s->ny;
     a.step = ROLE >= VAR_LAMBDA ? -(long long)plane : (long long)plane;
+    const bool odd = var_odd(s);
     BlockPlan plan{};
     if (nlevels > 0)
         plan = plan_var<ROLE>(BlockGrids{&grid, 1}, (int)std::min<int64_t>(nlevels, 1 << 20), sms);
@@ -630,7 +631,10 @@ int run_var(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t fra
                                        cudaMemcpyDeviceToDevice, s->stream));
         }
         if ((rc = timed_launch(s, 5, (double)plane * T,
-                               [&] { launch_var<ROLE>(a, T, sms, s->stream); })))
+                               [&] {
+                                   if (odd) launch_var<ROLE, true>(a, T, sms, s->stream);
+                                   else launch_var<ROLE>(a, T, sms, s->stream);
+                               })))
             return rc;
         s->cur = 1 - s->cur;
         done += T;
@@ -904,7 +908,7 @@ int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
     }
     if (s->eq == PS_EQ_EULER && s->threads != 256 && march_constants(make_params(s)))
         return run_march(s, nlevels, gts0, frames, frame_cap, frame_every, 5);
-    if (s->threads != 256 && var_aligned(s)) {
+    if (s->threads != 256) {
         if (s->eq == PS_EQ_HEATVAR && !s->field[1])
             return run_var<VAR_FORWARD>(s, nlevels, gts0, frames, frame_cap, frame_every);
         if (s->eq == PS_EQ_HEATVAR)
@@ -935,8 +939,7 @@ int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
     a.hx = s->bs / 2;
     a.Hmax = s->H;
     a.nb = s->nx / s->bs;
-    // (a count that does not divide ny was meant for blocks: one segment)
-    a.nseg = s->ny % s->nseg ? 1 : s->nseg;
+    a.nseg = s->nseg;
     a.wy = s->ny / a.nseg;
     a.nchunks = (a.wy + s->chunk - 1) / s->chunk;  // the last chunk may be partial
     a.seg_unit = a.wy;
