@@ -312,7 +312,7 @@ const char *ps_batch_last_error(const ps_batch *b);
  * ps_heatvar_forward: u_T after nsteps steps from u0.  Writes the courant
  * field to d_courant, uses d_work as scratch, and (if d_checkpoints != NULL)
  * stores u every `every` steps: checkpoint k = u_{k*every}, k = 0 ..
- * ceil(nsteps/every)-1.
+ * ceil(nsteps/every)-1.  d_uT may be d_u0.
  *
  * ps_heatvar_adjoint: for J(u_T) with d_lamT = dJ/du_T, writes dJ/du0 to
  * d_lam0 and dJ/dalpha to d_galpha, walking the checkpoint segments backward:

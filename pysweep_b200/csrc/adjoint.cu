@@ -187,10 +187,24 @@ extern "C" int ps_heatvar_forward(const double* d_u0, const double* d_alpha, dou
         done += len;
         if (d_checkpoints && done < nsteps) steps.back().ck = d_checkpoints + (size_t)(done / every) * n;
     }
+    auto out = [&](size_t k) {
+        return steps[k].ck ? steps[k].ck : ((steps.size() - 1 - k) % 2 == 0 ? d_uT : d_work);
+    };
     VarArgs a = var_args(d_courant, nx, ny);
     a.in = d_u0;
+    if (d_u0 == d_uT && out(0) == d_uT) {
+        // in place: tiles overlap, so no launch may write the field it reads
+        if (d_checkpoints) {
+            a.in = d_checkpoints;
+        } else {
+            if ((rc = adj_cuda(cudaMemcpyAsync(d_work, d_u0, n * sizeof(double), cudaMemcpyDeviceToDevice,
+                                               st), err, errlen)))
+                return rc;
+            a.in = d_work;
+        }
+    }
     for (size_t k = 0; k < steps.size(); ++k) {
-        a.out = steps[k].ck ? steps[k].ck : ((steps.size() - 1 - k) % 2 == 0 ? d_uT : d_work);
+        a.out = out(k);
         launch_var<VAR_FORWARD>(a, steps[k].T, sms, st);
         a.in = a.out;
     }
