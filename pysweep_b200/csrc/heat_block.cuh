@@ -153,9 +153,6 @@ __device__ __forceinline__ void block_store(S* row, int c0, int clo, int chi, in
 // ---------------------------------------------------------------- streams --
 // Exact columns of a strip.
 constexpr int kStreamC = 4, kStreamW = 32 * kStreamC - 2 * kStreamT;
-// Rows a strip steps besides its own: T above and below it, the last group's
-// delay, and the round to three steps.
-constexpr int kStreamRunIn = 2 * kStreamT + kStreamT / 2 - 1;
 
 // One strip: columns [cs vw, +vw), rows [x0, x1).  RK2: the levels alternate
 // half and full stage, starting with a half stage.
@@ -436,7 +433,7 @@ struct TileShape {
 // (eight and ten rows of four columns: grids whose tiles then fit the SMs in
 // fewer rounds, 1000 x 1400 1.73 -> 1.51 us per level, 1280² 1.95 -> 1.75)
 constexpr TileShape kTilesFE[] = {{4, 6, 16, 16}, {4, 6, 12, 16}, {4, 6, 8, 16},  {4, 8, 16, 16},
-                                  {4, 10, 12, 12}, {2, 8, 12, 20}, {2, 8, 8, 20}, {2, 8, 6, 20},
+                                  {4, 10, 12, 12}, {2, 8, 12, 20}, {2, 8, 8, 20},
                                   {2, 4, 12, 24}, {2, 4, 8, 24},  {2, 4, 6, 24},  {2, 4, 4, 24}};
 // Two stages keep two fields in registers.  us per level with four rows of four
 // columns and 16 warps, before / with these: 512² 0.95 / 0.60, 1120² 1.80 /

@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(32 * MAXW, 2) heatvar_back(const __grid_consta
 // rows and 10 warps.
 constexpr int kBackMaxT = 8;
 constexpr TileShape kTilesBack[] = {{2, 6, 8, 8}, {2, 6, 6, 8}, {2, 6, 4, 8},
-                                    {2, 4, 10, 10}, {2, 4, 8, 10}, {2, 4, 6, 10}};
+                                    {2, 4, 10, 10}, {2, 4, 8, 10}};
 
 // Estimated microseconds of one launch (fitted to launches of 256² to 2048²,
 // within 30%), or 0 where no cell of the tile stays exact.
