@@ -146,8 +146,8 @@ int ps_get_global_value(ps_solver *s, const char *name, double *value);
  * chunk = streaming chunk width (32 or 64) of the generic streams,
  * threads = 128 (default: overlapped blocks for heat, its per-cell-courant
  * forms and step hooks, Euler level by level) or 256 (always the shared-memory
- * prisms and seams).  A configured h also bounds the levels that a block runs
- * per launch.
+ * prisms and seams).  A configured h also bounds the levels that a block of heat
+ * or of a step hook runs per launch.
  * The defaults reproduce the reference's bs-row bands with MPSS levels per
  * half-cycle, except heat with forward Euler at bs 32 (12 levels); results do
  * not depend on the tiling.

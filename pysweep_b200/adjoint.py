@@ -200,9 +200,9 @@ class HeatVarSolve(torch.autograd.Function):
             courant = torch.empty_like(u0)
             _call(_lib.lib().ps_heatvar_courant, _p(alpha), _p(courant), nx, ny, dt, dx)
             form = "lambda" if swept == "lambda" else "mu"
-            # checkpoint segments of whole half-cycles (the values do not
-            # depend on the spacing; partial half-cycles cost a launch set
-            # for few levels)
+            # checkpoint segments of a multiple of the levels that the engine
+            # reports (the spacing decides how many fields the checkpoints and a
+            # segment's Laplacians take; the values do not depend on it)
             h = SweptHeatVar.levels_per_half_cycle(nx, ny, form, u0.device.index or 0)
             every = max(h, every - every % h)
             sw = _swept_solver(nx, ny, every, form, u0.device.index or 0)
