@@ -28,18 +28,20 @@
 namespace psb {
 namespace euler {
 
-// 1/b rounded correctly (y), and what is missing to 1/b (e).  Two steps of
-// Newton's method with fused multiply-adds, the first of third order, from an
-// approximation good to 2^-20 (the rcp.approx.ftz.f64 instruction): 2^-60, and
-// a last step that rounds correctly (P. Markstein, "Computation of elementary
-// functions on the IBM RISC System/6000 processor", 1990).  Take b in [1, 2), so
-// ulps of 1/b are 2^-53, and D the distance of 1/b from the nearest midpoint of
-// two doubles.  1 - b m is a nonzero multiple of 2^-106 for a midpoint m, so D
-// is at least 2^-53/b ulps.  The first step's result is off 1/b by at most
-// 1/2 + D ulps where D < 2^-7 (and by less than 0.51 elsewhere); the last
-// step's value before rounding is then off by b (1/2 + D)^2 2^-53 ulps, less than
-// D for every b but the largest, 2 - 2^-52, whose reciprocal comes out one ulp
-// low: its last bit is set here.
+// 1/b rounded correctly (y), and what is missing to 1/b (e).  From an
+// approximation y0 good to 2^-20 (the rcp.approx.ftz.f64 instruction), with r = 1 -
+// b y0: 1/b = y0/(1 - r), the geometric series y0 (1 + r + r^2 + ..) (M. J. Flynn,
+// "On division by functional iteration", IEEE Trans. Computers C-19, 1970), here
+// three terms of it by Horner's rule, good to 2^-60; then a step that rounds
+// correctly (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990).  Take b in [1, 2), so ulps of 1/b are 2^-53, and D
+// the distance of 1/b from the nearest midpoint of two doubles.  1 - b m is a
+// nonzero multiple of 2^-106 for a midpoint m, so D is at least 2^-53/b ulps.  The
+// series rounds a value within 2^-7 ulps of 1/b, so it is off by at most 1/2 + D
+// ulps where D < 2^-7 (and by less than 0.51 elsewhere); the last step's value
+// before rounding is then off by b (1/2 + D)^2 2^-53 ulps, less than D for every b
+// but the largest, 2 - 2^-52, whose reciprocal may come out one ulp low: its last
+// bit is set here.
 struct Recip {
     double b, y, e;
 };
@@ -47,8 +49,8 @@ __device__ __forceinline__ double recip_rn(double b)
 {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    const double t = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, __fma_rn(t, t, t), y);
+    const double r = __fma_rn(-b, y, 1.0), y1 = __fma_rn(y, r, y);
+    y = __fma_rn(y1, r, y);
     y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
     const unsigned ones = ((unsigned)__double2hiint(b) | 0xfff00000u) & (unsigned)__double2loint(b);
     return __hiloint2double(__double2hiint(y), __double2loint(y) | (ones == 0xffffffffu ? 1 : 0));
