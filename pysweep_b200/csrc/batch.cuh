@@ -9,7 +9,7 @@
 // the blocksize, so they share the levels per half-cycle and the shared-memory
 // layout.  The launches of a whole run are captured into one CUDA graph.
 // (Heat with forward Euler runs in the overlapped blocks' batched kernels,
-// heat_block.cuh.)
+// heat_block.cuh, Euler in the marching warps', euler_march.cuh.)
 #pragma once
 #include "swept.cuh"
 

@@ -18,7 +18,9 @@
 // result is the correctly rounded one, so levels equal the per-cell step's
 // (Euler::step) bitwise.  909 warp instructions per cell for the 1806 of tiles
 // with their faces in shared memory; G cells/s, tiles / here: 480² 6.6 / 11.4,
-// 1120² 8.8 / 18.7, 4096² 9.2 / 21.4.
+// 1120² 8.8 / 18.7, 4096² 9.2 / 21.4.  Rows with a value outside the safe ranges
+// below take plain divisions, as all do where a constant is: 480² 7.7, 1120² 10.4,
+// 2048² 12.5 (called instead of inline 6.0, 8.3, 9.3).
 #pragma once
 #include <cmath>
 
@@ -152,15 +154,6 @@ __device__ __forceinline__ void side(double gm1, const double* Q, double& p, dou
     ne = quot(__dmul_rn(__dadd_rn(Q[3], p), Q[A]), r);
 }
 
-// flux<DIR> and spectral<DIR> by the plain divisions.
-template <int DIR>
-__device__ __noinline__ void face_plain(double gamma, double gm1, const double* L, const double* R,
-                                        double* f, double* s)
-{
-    flux<DIR>(gm1, L, R, f);
-    spectral<DIR>(gamma, gm1, L, R, s);
-}
-
 // Two faces, each between cells a and b (q and the factor of the side towards
 // the face): flux f and spectral term s, the values of flux and spectral in
 // equations.cuh.  plain: some state of the warp's is out of the safe range.
@@ -181,21 +174,10 @@ __device__ __forceinline__ void faces2(bool plain, double gamma, double gm1,
             R[k][v] = __dsub_rn(qb[k][v], __dmul_rn(hb[k], d));  // + hb (qa - qb)
         }
     if (plain) {
-        // (copies: only this path's arrays live in local memory)
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-            double Lc[4], Rc[4], fc[4], sc[4];
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                Lc[v] = L[k][v];
-                Rc[v] = R[k][v];
-            }
-            face_plain<DIR>(gamma, gm1, Lc, Rc, fc, sc);
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                f[k][v] = fc[v];
-                s[k][v] = sc[v];
-            }
+            flux<DIR>(gm1, L[k], R[k], f[k]);
+            spectral<DIR>(gamma, gm1, L[k], R[k], s[k]);
         }
         return;
     }
@@ -251,7 +233,9 @@ struct MarchShared {
     double2 park[8][32];
 };
 
-// Strip `unit`: columns [cs kMarchW, +kMarchW), rows [rs hs, +hs).
+// Strip `unit`: columns [cs kMarchW, +kMarchW), rows [rs hs, +hs).  PLAIN: every row
+// takes the plain divisions (constants outside march_constants).
+template <bool PLAIN>
 __device__ __forceinline__ void march_body(const MarchArgs& a, int unit, MarchShared& sh)
 {
     auto& ring = sh.ring;
@@ -355,7 +339,7 @@ __device__ __forceinline__ void march_body(const MarchArgs& a, int unit, MarchSh
             double q[2][4], qn[2][4], f[2][4], t[2][4];
             cells(s, q);
             cells(s + 1, qn);
-            const bool plain = badc | badn | badl | badm;
+            const bool plain = PLAIN || (badc | badn | badl | badm);
             euler::faces2<1>(plain, gamma, gm1, q, qn, hl, hr, f, t);
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
@@ -377,7 +361,7 @@ __device__ __forceinline__ void march_body(const MarchArgs& a, int unit, MarchSh
             up[0] = lo[1] = __dsub_rn(Pc[1], Pc[0]);
             up[1] = __dsub_rn(__shfl_down_sync(0xffffffffu, Pc[0], 1), Pc[1]);
             lo[0] = __shfl_up_sync(0xffffffffu, up[1], 1);
-            const bool plain = limit2(lo, up, l, r) | badc;
+            const bool plain = limit2(lo, up, l, r) | badc | PLAIN;
             const double h[2] = {r[1], __shfl_down_sync(0xffffffffu, r[0], 1)};
             double q[2][4], qn[2][4], f[2][4], t[2][4];
             cells(s, q);
@@ -422,10 +406,11 @@ __device__ __forceinline__ void march_body(const MarchArgs& a, int unit, MarchSh
     }
 }
 
+template <bool PLAIN>
 __global__ void __launch_bounds__(32, kMarchWarps) euler_march(const __grid_constant__ MarchArgs a)
 {
     __shared__ __align__(16) MarchShared sh;
-    march_body(a, blockIdx.x, sh);
+    march_body<PLAIN>(a, blockIdx.x, sh);
 }
 
 // Many instances in one launch: block g is unit units[g].y of instance
@@ -437,6 +422,7 @@ struct MarchInst {
     int nx, ny, level;
 };
 
+template <bool PLAIN>
 __global__ void __launch_bounds__(32, kMarchWarps)
     euler_march_batch(const MarchInst* __restrict__ inst, const int2* __restrict__ units, int cur,
                       int prev, int out, int hs, int L)
@@ -459,7 +445,7 @@ __global__ void __launch_bounds__(32, kMarchWarps)
     a.dtdy = b.dtdy;
     a.gamma = b.gamma;
     a.gm1 = b.gm1;
-    march_body(a, u.y, sh);
+    march_body<PLAIN>(a, u.y, sh);
 }
 
 // Rows of a strip: the fewest that fit one wave of warps, or 6 to 24 in several
@@ -501,7 +487,8 @@ inline int march_rows(const BlockGrids& g, int sms)
     return best;
 }
 
-// The constants for which the safe ranges above hold.
+// The constants for which the safe ranges above hold; with others every row takes
+// the plain divisions.
 inline bool march_constants(const EqParams& p)
 {
     auto mid = [](double x) { return x >= 0x1p-20 && x <= 0x1p20; };

@@ -709,6 +709,7 @@ int run_march(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
     a.dtdy = prm.d[1];
     a.gamma = prm.d[2];
     a.gm1 = prm.d[3];
+    const auto kernel = march_constants(prm) ? euler_march<false> : euler_march<true>;
     const int units = a.ncs * ((s->nx + a.hs - 1) / a.hs);
     return run_levels(s, nlevels, gts0, frames, frame_cap, frame_every, kind,
                       [&](const double* cur, const double* prev, double* out, double* fr, int gts) {
@@ -717,7 +718,7 @@ int run_march(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
                           a.out = out;
                           a.frame = fr;
                           a.gts = gts;
-                          launch_after(euler_march, units, 32, 0, s->stream, a);
+                          launch_after(kernel, units, 32, 0, s->stream, a);
                       });
 }
 
@@ -906,7 +907,7 @@ int run_swept(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_t f
         const HookBlock b = solver_hook_block(s, s->h_set ? s->H : kHookBlkMaxT);
         if (b.rows) return run_hook_block(s, b, nlevels, gts0, frames, frame_cap, frame_every);
     }
-    if (s->eq == PS_EQ_EULER && s->threads != 256 && march_constants(make_params(s)))
+    if (s->eq == PS_EQ_EULER && s->threads != 256)
         return run_march(s, nlevels, gts0, frames, frame_cap, frame_every, 5);
     if (s->threads != 256) {
         if (s->eq == PS_EQ_HEATVAR && !s->field[1])
@@ -1018,7 +1019,7 @@ int run_standard(ps_solver* s, int64_t nlevels, int gts0, double* frames, int64_
     StdLaunch K = s->hook ? nullptr : pick_standard(s->eq, s->ops);
     if (!K && !s->hook) return fail(s, PS_ERR_UNSUPPORTED, "no standard kernel for equation %d", s->eq);
     // (threads = 256 keeps the per-cell kernels)
-    if (s->eq == PS_EQ_EULER && s->threads != 256 && march_constants(make_params(s)))
+    if (s->eq == PS_EQ_EULER && s->threads != 256)
         return run_march(s, nlevels, gts0, frames, frame_cap, frame_every, 4);
     if (s->eq == PS_EQ_HEAT && s->threads != 256) {
         const bool fwd = make_params(s).i[0] != 0;
@@ -1899,15 +1900,6 @@ size_t batch_seam_smem(const ps_batch* b)
                                      seam_smem_elems(true, b->bs, b->ops, b->nv, b->its, b->H));
 }
 
-using BatchGen = void (*)(const SweptArgs*, const int2*, int, int, long long);
-
-struct BatchKernels {
-    const void* P = nullptr;
-    const void* G = nullptr;
-    const void* Y = nullptr;
-    const void* O = nullptr;
-};
-
 // Enqueue one half-cycle for every instance: P, then Y on the batch stream
 // beside G on the side stream (G reads nothing Y writes; see run_swept), then
 // O after both.
@@ -1954,11 +1946,11 @@ bool batch_pick(int eq, int ops, int its, int chunk, HalfFn* half, PrepFn* prep)
     }
     PS_BSET(PS_EQ_HEAT, 1, 1, 32, Heat)
     PS_BSET(PS_EQ_HEAT, 1, 2, 32, Heat)
-    PS_BSET(PS_EQ_EULER, 2, 2, 32, Euler)
-    PS_BSET(PS_EQ_EULER, 2, 2, 64, Euler)
     PS_BSET(PS_EQ_HALF, 1, 2, 32, Half)
 #undef PS_BSET
-    return false;
+    *half = nullptr;  // Euler runs level by level
+    *prep = nullptr;
+    return eq == PS_EQ_EULER && ops == 2 && its == 2;
 }
 
 // ---- heat in overlapped blocks (b->fast) ----
@@ -2073,14 +2065,6 @@ int batch_block_enqueue(ps_batch* b, const std::vector<BlockStep>& steps)
 }
 
 // ---- Euler level by level ----
-bool batch_marches(const ps_batch* b)
-{
-    if (b->eq != PS_EQ_EULER) return false;
-    for (const auto& I : b->inst)
-        if (!march_constants(make_params_g(b->eq, I.globals))) return false;
-    return true;
-}
-
 int batch_march_upload(ps_batch* b)
 {
     std::vector<MarchInst> d;
@@ -2110,10 +2094,13 @@ int batch_march_plan(ps_batch* b, int* hs, int* table)
 int batch_march_enqueue(ps_batch* b, int64_t nlevels, int hs, int table)
 {
     const ps_batch::Table& t = b->tables[table];
+    bool safe = true;  // (one kernel for all instances)
+    for (const auto& I : b->inst) safe = safe && march_constants(make_params_g(b->eq, I.globals));
+    const auto kernel = safe ? euler_march_batch<false> : euler_march_batch<true>;
     int older = 2 * b->cur, newest = older + 1;  // as in run_levels
     for (int64_t L = 1; L <= nlevels; ++L) {
         const int next = (newest + 1) % 4;
-        launch_after(euler_march_batch, t.n, 32, 0, b->stream, (const MarchInst*)b->d_minst,
+        launch_after(kernel, t.n, 32, 0, b->stream, (const MarchInst*)b->d_minst,
                      (const int2*)t.d, newest, older, next, hs, (int)L);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return bfail(b, PS_ERR_CUDA, "batched launch: %s", cudaGetErrorString(e));
@@ -2192,11 +2179,6 @@ int ps_batch_create(ps_batch** out, int device, int equation, int count, const i
     b->mpss = blocksize / (2 * ops) - 1;
     b->H = default_levels(equation, its, blocksize, b->mpss);
     b->fast = equation == PS_EQ_HEAT && its == 1 && (blocksize == 16 || blocksize == 32);
-    // Euler: 64-column chunks where the tile fits (as for a solver)
-    if (!b->fast && equation == PS_EQ_EULER) {
-        b->chunk = 64;
-        if (batch_tile_smem(b) > 227 * 1024) b->chunk = 32;
-    }
     int rc = PS_OK;
     std::vector<int2> units;
     for (int i = 0; i < count && rc == PS_OK; ++i) {
@@ -2249,9 +2231,10 @@ int ps_batch_create(ps_batch** out, int device, int equation, int count, const i
         I.yface_n = yn;
         cudaError_t e = cudaMalloc(&I.base[0], f * its * sizeof(double));
         if (e == cudaSuccess) e = cudaMalloc(&I.base[1], f * its * sizeof(double));
-        // (the overlapped blocks keep no faces)
-        if (e == cudaSuccess && xn && !b->fast) e = cudaMalloc(&I.xface, xn * sizeof(double));
-        if (e == cudaSuccess && yn && !b->fast) e = cudaMalloc(&I.yface, yn * sizeof(double));
+        // (blocks and single levels keep no faces)
+        const bool faces = !b->fast && equation != PS_EQ_EULER;
+        if (e == cudaSuccess && xn && faces) e = cudaMalloc(&I.xface, xn * sizeof(double));
+        if (e == cudaSuccess && yn && faces) e = cudaMalloc(&I.yface, yn * sizeof(double));
         if (e != cudaSuccess) rc = bfail(b, PS_ERR_NOMEM, "instance buffers: %s", cudaGetErrorString(e));
     }
     if (rc == PS_OK) {
@@ -2271,7 +2254,7 @@ int ps_batch_create(ps_batch** out, int device, int equation, int count, const i
     // the kernels of the chosen chunk width (prep opts them into large shared memory)
     if (rc == PS_OK && !batch_pick(equation, ops, its, b->chunk, &half, &prep))
         rc = bfail(b, PS_ERR_UNSUPPORTED, "no batched kernels for chunk %d", b->chunk);
-    if (rc == PS_OK) prep();
+    if (rc == PS_OK && prep) prep();
     if (rc != PS_OK) {
         g_create_error = b->err;
         ps_batch_destroy(b);
@@ -2363,7 +2346,7 @@ int ps_batch_run(ps_batch* b, int64_t nlevels, int use_graph)
         nsteps = b->graph_launches;
     }
     // Euler: base buffers of two levels each, one launch per level
-    const bool march = batch_marches(b);
+    const bool march = b->eq == PS_EQ_EULER;
     int hs = 0, table = 0;
     if (march) {
         nsteps = (nlevels + 1) / 2;  // (the newest level's base buffer changes every other level)
