@@ -156,9 +156,9 @@ __device__ __forceinline__ void side(double gm1, const double* Q, double& p, dou
 
 // Two faces, each between cells a and b (q and the factor of the side towards
 // the face): flux f and spectral term s, the values of flux and spectral in
-// equations.cuh.  plain: some state of the warp's is out of the safe range.
-template <int DIR>
-__device__ __forceinline__ void faces2(bool plain, double gamma, double gm1,
+// equations.cuh.  PLAIN: some state of the warp's is out of the safe range.
+template <int DIR, bool PLAIN>
+__device__ __forceinline__ void faces2(double gamma, double gm1,
                                        const double (&qa)[2][4], const double (&qb)[2][4],
                                        const double (&ha)[2], const double (&hb)[2],
                                        double (&f)[2][4], double (&s)[2][4])
@@ -173,7 +173,7 @@ __device__ __forceinline__ void faces2(bool plain, double gamma, double gm1,
             L[k][v] = __dadd_rn(qa[k][v], __dmul_rn(ha[k], d));
             R[k][v] = __dsub_rn(qb[k][v], __dmul_rn(hb[k], d));  // + hb (qa - qb)
         }
-    if (plain) {
+    if constexpr (PLAIN) {
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             flux<DIR>(gm1, L[k], R[k], f[k]);
@@ -226,7 +226,7 @@ struct MarchArgs {
 };
 
 // A warp's shared memory: rows of the strip, and what a row's face phase
-// leaves for later: [0..3] its derivative terms along x, [4..7] flux + spectral
+// leaves for later: [0..3] its flux differences along x, [4..7] flux + spectral
 // term of the face below the next row.
 struct MarchShared {
     double ring[kMarchRing][4][64];
@@ -249,7 +249,7 @@ __device__ __forceinline__ void march_body(const MarchArgs& a, int unit, MarchSh
     const int g = wrap(c0, ny);
     const size_t plane = (size_t)nx * ny;
     const double gamma = a.gamma, gm1 = a.gm1;
-    const double hx = 0.5 * a.dtdx, hy = 0.5 * a.dtdy;  // (the fluxes' factor 1/2 scales exactly)
+    const double hx = 0.5 * a.dtdx, hy = 0.5 * a.dtdy;
     const bool full = a.gts % 2 == 0;
     const bool mine = c0 >= clo && c0 < chi;
     const int n = x1 - x0 + 4;  // rows read: x0-2 .. x1+1
@@ -302,7 +302,7 @@ __device__ __forceinline__ void march_body(const MarchArgs& a, int unit, MarchSh
     // factor of row i towards its upper face; badc, badn: unsafe rows; badl:
     // unsafe factors of row i
     double Pc[2], Pn[2], dn[2], hl[2];
-    bool badc, badn, badl;
+    bool badc, badn, badl, below = false;  // below: `above` of the row before
     {
         double Pm[2], dm[2], unused[2];
         pressures(0, Pm);
@@ -335,19 +335,20 @@ __device__ __forceinline__ void march_body(const MarchArgs& a, int unit, MarchSh
 #pragma unroll
         for (int k = 0; k < 2; ++k) df[k] = __dsub_rn(Pf[k], Pn[k]);
         const bool badm = limit2(dn, df, hn, hr);
+        const bool above = PLAIN || (badc | badn | badl | badm);  // plain divisions for the face above row i
         {
             double q[2][4], qn[2][4], f[2][4], t[2][4];
             cells(s, q);
             cells(s + 1, qn);
-            const bool plain = PLAIN || (badc | badn | badl | badm);
-            euler::faces2<1>(plain, gamma, gm1, q, qn, hl, hr, f, t);
+            if (above) euler::faces2<1, true>(gamma, gm1, q, qn, hl, hr, f, t);
+            else euler::faces2<1, false>(gamma, gm1, q, qn, hl, hr, f, t);
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
                 const double2 lo = park[4 + v][lane];
                 double D[2], G[2];
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
-                    D[k] = __dmul_rn(__dsub_rn(__dsub_rn(k ? lo.y : lo.x, f[k][v]), t[k][v]), hx);
+                    D[k] = __dsub_rn(__dsub_rn(k ? lo.y : lo.x, f[k][v]), t[k][v]);
                     G[k] = __dadd_rn(__dadd_rn(0.0, f[k][v]), t[k][v]);
                 }
                 park[v][lane] = make_double2(D[0], D[1]);
@@ -361,28 +362,44 @@ __device__ __forceinline__ void march_body(const MarchArgs& a, int unit, MarchSh
             up[0] = lo[1] = __dsub_rn(Pc[1], Pc[0]);
             up[1] = __dsub_rn(__shfl_down_sync(0xffffffffu, Pc[0], 1), Pc[1]);
             lo[0] = __shfl_up_sync(0xffffffffu, up[1], 1);
-            const bool plain = limit2(lo, up, l, r) | badc | PLAIN;
+            const bool plain = limit2(lo, up, l, r) | badc | above | below;
             const double h[2] = {r[1], __shfl_down_sync(0xffffffffu, r[0], 1)};
-            double q[2][4], qn[2][4], f[2][4], t[2][4];
+            double q[2][4], qn[2][4], o[2][4];
             cells(s, q);
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
                 qn[0][v] = q[1][v];
                 qn[1][v] = ring[s % kMarchRing][v][min(2 * lane + 2, 63)];
             }
-            euler::faces2<2>(plain, gamma, gm1, q, qn, l, h, f, t);
-            double o[2][4];
+            // The stage: u + d/2 or the level before + d, d = (dx/2) dt/dx + (dy/2)
+            // dt/dy of the flux differences dx, dy.  Of states in the safe ranges no
+            // difference and no d is subnormal, so halving them is exact: it goes into
+            // dt/dx and into a fused multiply-add.  (us per level at 1120²: so in every
+            // row, which is wrong, 67.2; an arm for the other rows 67.8; a branch of
+            // their own behind the faces 68.3.)
+            auto row = [&](auto slow) {
+                constexpr bool SLOW = decltype(slow)::value;
+                double f[2][4], t[2][4];
+                euler::faces2<2, SLOW>(gamma, gm1, q, qn, l, h, f, t);
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                const double gi = __dadd_rn(__dadd_rn(0.0, f[0][v]), t[0][v]);
-                const double gl = __shfl_up_sync(0xffffffffu, __dadd_rn(__dadd_rn(0.0, f[1][v]), t[1][v]), 1);
-                const double e0 = __dmul_rn(__dsub_rn(__dsub_rn(gl, f[0][v]), t[0][v]), hy);
-                const double e1 = __dmul_rn(__dsub_rn(__dsub_rn(gi, f[1][v]), t[1][v]), hy);
-                const double2 D = park[v][lane];
-                const double d0 = __dadd_rn(D.x, e0), d1 = __dadd_rn(D.y, e1);
-                o[0][v] = full ? __dadd_rn(pv[v].x, d0) : __fma_rn(0.5, d0, q[0][v]);
-                o[1][v] = full ? __dadd_rn(pv[v].y, d1) : __fma_rn(0.5, d1, q[1][v]);
-            }
+                for (int v = 0; v < 4; ++v) {
+                    const double gi = __dadd_rn(__dadd_rn(0.0, f[0][v]), t[0][v]);
+                    const double gl =
+                        __shfl_up_sync(0xffffffffu, __dadd_rn(__dadd_rn(0.0, f[1][v]), t[1][v]), 1);
+                    const double2 D = park[v][lane];
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const double x = k ? D.y : D.x, y = __dsub_rn(__dsub_rn(k ? gi : gl, f[k][v]), t[k][v]);
+                        const double d = SLOW ? __dadd_rn(__dmul_rn(__dmul_rn(x, 0.5), a.dtdx),
+                                                          __dmul_rn(__dmul_rn(y, 0.5), a.dtdy))
+                                              : __dadd_rn(__dmul_rn(x, hx), __dmul_rn(y, hy));
+                        if (full) o[k][v] = __dadd_rn(k ? pv[v].y : pv[v].x, d);
+                        else o[k][v] = SLOW ? __dadd_rn(q[k][v], __dmul_rn(0.5, d)) : __fma_rn(0.5, d, q[k][v]);
+                    }
+                }
+            };
+            if (PLAIN || plain) row(std::true_type());
+            else row(std::false_type());
             if (mine) {
 #pragma unroll
                 for (int v = 0; v < 4; ++v) {
@@ -403,6 +420,7 @@ __device__ __forceinline__ void march_body(const MarchArgs& a, int unit, MarchSh
         badc = badn;
         badn = badf;
         badl = badm;
+        below = above;
     }
 }
 

@@ -11,13 +11,25 @@ from test_gpu_euler_march import G, _field, _state
 pytestmark = pytest.mark.gpu
 
 
-def _subnormal(nx, ny, axis):
-    """Uniform flow along one axis, momenta of 1 to 2^24 times the smallest
-    subnormal across it: their flux differences are odd multiples of it, too."""
-    rng = np.random.default_rng([nx, ny, axis])
-    one = np.ones((nx, ny))
+def _subnormal(nx, ny, kind):
+    """Uniform flow along one axis, momenta of multiples of the smallest subnormal
+    across it, so that their flux differences are odd multiples of it, too: 1 to
+    2^24 of them, a few of either sign and zeros of both, or those in a few rows
+    and columns only."""
+    rng = np.random.default_rng([nx, ny, len(kind)])
+    one, axis = np.ones((nx, ny)), int(kind[-1])
     q = _state(one, one if axis == 0 else 0 * one, one if axis == 1 else 0 * one, one)
-    q[2 if axis == 0 else 1] = rng.integers(1, 1 << 24, (nx, ny)) * 2.0 ** -1074
+    many = rng.integers(1, 1 << 24, (nx, ny)) * 2.0 ** -1074
+    few = rng.choice([-3.0, -2.0, -1.0, -0.0, 0.0, 1.0, 2.0, 3.0], (nx, ny)) * 2.0 ** -1074
+    if kind.startswith("many"):
+        v = many
+    elif kind.startswith("few"):
+        v = few
+    else:
+        v = np.full((nx, ny), -0.0)
+        for at in ((10, slice(None)), (11, slice(30, 34)), (57, slice(0, 3)), (slice(40, 44), 70)):
+            v[at] = few[at]
+    q[2 if axis == 0 else 1] = v
     return q
 
 
@@ -38,10 +50,11 @@ def _bits(a):
     return np.ascontiguousarray(a).view(np.int64)
 
 
-@pytest.mark.parametrize("kind", ["vortex", "uniform", "steps", "below_two", "jumps", "subnormal0", "subnormal1"])
+@pytest.mark.parametrize("kind", ["vortex", "uniform", "steps", "below_two", "jumps", "many0", "many1", "few0", "few1",
+                                  "some0", "some1"])
 @pytest.mark.parametrize("nl", [1, 2, 7])
 def test_march_has_the_per_cell_bits(kind, nl):
-    ic = _subnormal(96, 128, int(kind[-1])) if kind[:-1] == "subnormal" else _field(kind, 96, 128)
+    ic = _subnormal(96, 128, kind) if kind[-1] in "01" else _field(kind, 96, 128)
     ref = _solve(ic, nl, "standard", threads=256)
     for mode in ("swept", "standard"):
         for a, b in zip(_solve(ic, nl, mode), ref):
