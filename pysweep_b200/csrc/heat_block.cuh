@@ -19,8 +19,9 @@
 //       takes one new row and computes one row of every level.  The levels
 //       run in groups of two, each group one row behind the one before it, so
 //       a step holds four independent chains instead of one of eight (8192²:
-//       346 -> 329 us per 8 levels).  112 of the 128 columns are exact at the
-//       end (12.5% evaluated twice).
+//       346 -> 329 us per 8 levels, the kernel alone; 339 in a run's row of
+//       launches, 367 once a long one has met the 1000 W cap).  112 of the 128
+//       columns are exact at the end (12.5% evaluated twice).
 //   heat_block_tile    A CTA holds a tile of nw x R rows and 32 C columns in
 //       registers and steps it in place, neighbouring warps exchanging one
 //       row each way per level through shared memory.  Rows of a warp are
@@ -560,8 +561,8 @@ inline BlockPlan plan_tiles(const TileShape (&shapes)[NSHAPE], const BlockGrids&
 }
 
 // The cheapest way to run nlevels levels.  Streams win from about 2000² up
-// (us per level, stream / best tile: 1120² 2.08 / 1.33, 2048² 4.02 / 4.05,
-// 4096² 11.6 / 15.7, 8192² 42.4 / 60.0); below, the tile whose count fits the
+// (us per level in runs of 480, stream / best tile: 1120² 2.08 / 1.33, 2048² 4.02 /
+// 4.05, 4096² 11.6 / 15.7, 8192² 42.4 / 60.0); below, the tile whose count fits the
 // SMs best.
 template <int NSHAPE>
 inline BlockPlan plan_block(const TileShape (&shapes)[NSHAPE], const BlockGrids& g, int nlevels,
