@@ -16,7 +16,7 @@
 // operations on it (quot); a cell's two limiter ratios are each other's inverse,
 // and one of them needs no value but whether it exceeds 1e6 (limiters).  Every
 // result is the correctly rounded one, so levels equal the per-cell step's
-// (Euler::step) bitwise.  909 warp instructions per cell for the 1806 of tiles
+// (Euler::step) bitwise.  907 warp instructions per cell for the 1806 of tiles
 // with their faces in shared memory; G cells/s, tiles / here: 480² 6.6 / 11.3,
 // 1120² 8.8 / 18.5, 4096² 9.2 / 22.3.  Rows with a value outside the safe ranges
 // below take plain divisions, as all do where a constant is: 480² 7.7, 1120² 10.4,

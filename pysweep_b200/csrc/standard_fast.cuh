@@ -8,7 +8,7 @@
 // shuffle (lanes 0 and 31 load theirs).  Arithmetic: Heat in equations.cuh.
 // Bound by HBM where the fields exceed L2 (16 bytes per cell: 428 G cells/s at
 // 8192² in a short run, 106% of the measured copy's rate, the halo rows coming from
-// L2; 404 in one of 5000 levels), below
+// L2; 405 in one of 5000 levels), below
 // by the launch and one round trip.  us per level, against rows streamed one by
 // one down 32-row strips: 2048² 14.4 -> 7.2, 4096² 49 -> 41, 8192² 182 -> 157;
 // against one thread per cell (1120 columns are no multiple of 64): 7.4 -> 3.3.
